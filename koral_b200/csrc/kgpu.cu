@@ -1017,8 +1017,7 @@ __device__ inline int u2p_run(const Grid &G, int Etype, U2PCell &x, int stop, do
   u2p_setup(x.uc, x.g, st);
   W = u2p_initial_w(G.gamma, x.pp, x.g);
   iter = 0;
-  if (u2p_bracket(G.gamma, Etype, st.c, W)) return -150;
-  int r = u2p_newton(G.gamma, G.u2pconv, Etype, st.c, W, iter, stop, U2P_DAMP_BUDGET);
+  const int r = u2p_solve_w(G.gamma, G.u2pconv, Etype, st.c, W, iter, stop, U2P_DAMP_BUDGET);
   if (r) return r;
   return u2p_final(G.gamma, st, W, iter, x.uc, x.pp, x.g);
 }

@@ -511,15 +511,107 @@ KG_HD double u2p_initial_w(double GAMMA, const double *pp, const Geom &g) {
   return (pp[0] + GAMMA * pp[1]) * gamma2;
 }
 
-// W x 10 until the state is physical (u2p.c:2117-2135); 0 or -150
-KG_HD int u2p_bracket(double GAMMA, int Etype, const U2PCons &c, double &W, unsigned *fevals = nullptr) {
-  double f0, dfdW, err;
+constexpr int U2P_PAUSED = 1;
+// returned by a capped W solve that used up its function evaluations (the
+// caller repeats the whole inversion another way; nothing is kept)
+constexpr int U2P_OVER_CAP = 7;
+
+// The W function at one point.
+struct U2PF {
+  double f, df, err;
+};
+
+// The W solve: W x 10 until the state is physical (u2p.c:2117-2135), then
+// Newton iterations (u2p.c:2140-2200) until convergence, failure, or a
+// pause: at the top of an iteration once iter reaches `stop`, or before an
+// iteration whose damped step would need `damp_budget` or more halvings
+// (the iteration is then undone, (W, iter) as before it).  A paused solve
+// that is resumed (u2p_newton_warp) takes exactly the steps an
+// uninterrupted one takes.  Returns 0 when the loop has ended (the caller
+// finishes with u2p_final), U2P_PAUSED, or a negative reference status on
+// failure.
+//
+// The reference evaluates the function again at the top of every iteration,
+// at the W where the bracketing or the accepted trial of the iteration before
+// has just evaluated it.  Here that value is carried over, which halves the
+// evaluations of a typical solve (four to two when it converges in two
+// steps), and bracketing and trials share one copy of the function in the
+// instruction stream, in which the lanes of a warp meet whatever each of
+// them is doing.  `fevals` still counts the evaluations of the reference's
+// sequence, so the limit `fcap` acts where it did.
+KG_HD int u2p_solve_w(double GAMMA, double CONV, int Etype, const U2PCons &c, double &W, int &iter, int stop,
+                      int damp_budget = 1 << 30, unsigned *fevals = nullptr, unsigned fcap = 0) {
+  enum { BRACKET, TRIAL, AGAIN };      // why the function is evaluated at `at`
+  int mode = BRACKET;
+  int n = 0;                           // bracketing steps, then halvings of the running step
+  double at = W, dumpfac = 1.;
+  U2PF F, S{0., 0., 0.};               // the last evaluation; the one the running step started from
+  while (true) {
+    f_u2p(GAMMA, Etype, at - c.D, c, F.f, F.df, F.err);
+    if (mode != AGAIN) {
+      if (fevals) (*fevals)++;
+      const bool bad = u2p_bad_w(at, c.Bsq, c.QdotBsq, c.Qt2, F.f, F.df);
+      if (mode == BRACKET) {
+        if (bad && n < 50) {
+          W *= 10.;
+          at = W;
+          n++;
+          continue;
+        }
+        if (n >= 50) return -150;
+      } else {
+        if (bad && n < 100) {
+          if (fcap && *fevals >= fcap) return U2P_OVER_CAP;
+          n++;
+          if (n >= damp_budget) {
+            iter--;
+            return U2P_PAUSED;
+          }
+          dumpfac /= 2.;
+          at = W - dumpfac * S.f / S.df;
+          continue;
+        }
+        if (n >= 100) return -101;
+        const double Wprev = W;
+        W = at;
+        if (fabs(W) > BIG) return -103;
+        if (fabs((W - Wprev) / Wprev) < CONV && S.err < 1.e-1) return 0;
+        if (!(iter < 50)) return 0;
+      }
+      // top of an iteration, the function known at W
+      if (iter >= stop && iter < 50) return U2P_PAUSED;
+      if (fcap && *fevals >= fcap) return U2P_OVER_CAP;
+      iter++;
+      if (fevals) (*fevals)++;
+    }
+    if (F.err < CONV) return 0;
+    if (F.df == 0.) {
+      W *= 1.1;
+      if (!(iter < 50)) return 0;
+      if (iter >= stop && iter < 50) return U2P_PAUSED;
+      if (fcap && *fevals >= fcap) return U2P_OVER_CAP;
+      iter++;
+      if (fevals) (*fevals)++;
+      mode = AGAIN;
+      at = W;
+      continue;
+    }
+    S = F;
+    mode = TRIAL;
+    n = 0;
+    dumpfac = 1.;
+    at = W - S.f / S.df;
+  }
+}
+
+// W x 10 until the state is physical (u2p.c:2117-2135), and the function at
+// the W found; 0 or -150
+KG_HD int u2p_bracket(double GAMMA, int Etype, const U2PCons &c, double &W, U2PF &F, unsigned *fevals = nullptr) {
   int i_increase = 0;
   while (true) {
-    f0 = dfdW = 0.;
     if (fevals) (*fevals)++;
-    f_u2p(GAMMA, Etype, W - c.D, c, f0, dfdW, err);
-    if (u2p_bad_w(W, c.Bsq, c.QdotBsq, c.Qt2, f0, dfdW) && (i_increase < 50)) {
+    f_u2p(GAMMA, Etype, W - c.D, c, F.f, F.df, F.err);
+    if (u2p_bad_w(W, c.Bsq, c.QdotBsq, c.Qt2, F.f, F.df) && (i_increase < 50)) {
       W *= 10.;
       i_increase++;
       continue;
@@ -529,117 +621,68 @@ KG_HD int u2p_bracket(double GAMMA, int Etype, const U2PCons &c, double &W, unsi
   return i_increase >= 50 ? -150 : 0;
 }
 
-constexpr int U2P_PAUSED = 1;
-// returned by a capped W solve that used up its function evaluations (the
-// caller repeats the whole inversion another way; nothing is kept)
-constexpr int U2P_OVER_CAP = 7;
-
-// Newton iterations (u2p.c:2140-2200) until convergence, failure, or a
-// pause: at the top of an iteration once iter reaches `stop`, or before an
-// iteration whose damped step would need `damp_budget` or more halvings
-// (the iteration is then undone, (W, iter) as before it).  A paused solve
-// resumed with larger limits takes exactly the steps an uninterrupted one
-// takes.  Returns 0 when the loop has ended (the caller finishes with
-// u2p_final), U2P_PAUSED, or a negative reference status on failure.
-KG_HD int u2p_newton(double GAMMA, double CONV, int Etype, const U2PCons &c, double &W, int &iter, int stop,
-                     int damp_budget = 1 << 30, unsigned *fevals = nullptr, unsigned fcap = 0) {
-  const double D = c.D;
-  double f0, dfdW, err;
-  while (true) {
-    if (iter >= stop && iter < 50) return U2P_PAUSED;
-    if (fcap && *fevals >= fcap) return U2P_OVER_CAP;
-    double Wprev = W;
-    iter++;
-    if (fevals) (*fevals)++;
-    f_u2p(GAMMA, Etype, W - D, c, f0, dfdW, err);
-    if (err < CONV) break;
-    if (dfdW == 0.) {
-      W *= 1.1;
-      if (iter < 50) continue;
-      break;
-    }
-    double Wnew = W - f0 / dfdW;
-    int idump = 0;
-    double dumpfac = 1.;
-    while (true) {
-      double f0t = 0., dft = 0., errt;
-      if (fevals) (*fevals)++;
-      f_u2p(GAMMA, Etype, Wnew - D, c, f0t, dft, errt);
-      if (u2p_bad_w(Wnew, c.Bsq, c.QdotBsq, c.Qt2, f0t, dft) && (idump < 100)) {
-        if (fcap && *fevals >= fcap) return U2P_OVER_CAP;
-        idump++;
-        if (idump >= damp_budget) {
-          W = Wprev;
-          iter--;
-          return U2P_PAUSED;
-        }
-        dumpfac /= 2.;
-        Wnew = W - dumpfac * f0 / dfdW;
-        continue;
-      }
-      break;
-    }
-    if (idump >= 100) return -101;
-    W = Wnew;
-    if (fabs(W) > BIG) return -103;
-    if (fabs((W - Wprev) / Wprev) < CONV && err < 1.e-1) break;
-    if (!(iter < 50)) break;
-  }
-  return 0;
-}
-
 #ifdef __CUDACC__
 // The same iterations carried out by a whole warp on one cell (all lanes
 // hold the same state): the damped step's trial points, which the scalar
 // loop tries one after another, are tried 32 at a time and the first
 // acceptable one is taken.  Trial k is W - 2^-k f/f' as in the scalar loop
 // (2^-k is the exact result of its repeated halving), so the result is the
-// same bit for bit.  Every lane returns the same values.
-__device__ inline int u2p_newton_warp(double GAMMA, double CONV, int Etype, const U2PCons &c, double &W, int &iter) {
+// same bit for bit.  Every lane returns the same values.  F: the function at
+// the incoming W where the caller has it (have); the accepted trial's
+// evaluation is passed on to the next iteration by shuffles instead of being
+// done again, which halves the chain of dependent evaluations.
+__device__ inline int u2p_newton_warp(double GAMMA, double CONV, int Etype, const U2PCons &c, double &W, int &iter,
+                                      U2PF F = U2PF{0., 0., 0.}, bool have = false) {
   const int lane = threadIdx.x & 31;
   const double D = c.D;
-  double f0, dfdW, err;
   while (true) {
     double Wprev = W;
     iter++;
-    f_u2p(GAMMA, Etype, W - D, c, f0, dfdW, err);
-    if (err < CONV) break;
-    if (dfdW == 0.) {
+    if (!have) f_u2p(GAMMA, Etype, W - D, c, F.f, F.df, F.err);
+    have = false;
+    if (F.err < CONV) break;
+    if (F.df == 0.) {
       W *= 1.1;
       if (iter < 50) continue;
       break;
     }
     double Wnew = 0.;
+    U2PF Fn = F;
     int found = -1;
     for (int base = 0; base <= 100 && found < 0; base += 32) {
       const int k = base + lane;
       double Wk = 0.;
+      U2PF T{0., 0., 0.};
       bool accept = false;
       if (k == 0) {
-        Wk = W - f0 / dfdW;
+        Wk = W - F.f / F.df;
       } else if (k <= 100) {
         const double dumpfac = ldexp(1.0, -k);
-        Wk = W - dumpfac * f0 / dfdW;
+        Wk = W - dumpfac * F.f / F.df;
       }
       if (k == 100) {
         accept = true;   // the scalar loop stops here whatever the state
       } else if (k < 100) {
-        double f0t = 0., dft = 0., errt;
-        f_u2p(GAMMA, Etype, Wk - D, c, f0t, dft, errt);
-        accept = !u2p_bad_w(Wk, c.Bsq, c.QdotBsq, c.Qt2, f0t, dft);
+        f_u2p(GAMMA, Etype, Wk - D, c, T.f, T.df, T.err);
+        accept = !u2p_bad_w(Wk, c.Bsq, c.QdotBsq, c.Qt2, T.f, T.df);
       }
       const unsigned m = __ballot_sync(0xffffffffu, accept);
       if (m) {
         const int L = __ffs(m) - 1;
         found = base + L;
         Wnew = __shfl_sync(0xffffffffu, Wk, L);
+        Fn.f = __shfl_sync(0xffffffffu, T.f, L);
+        Fn.df = __shfl_sync(0xffffffffu, T.df, L);
+        Fn.err = __shfl_sync(0xffffffffu, T.err, L);
       }
     }
     if (found >= 100) return -101;
     W = Wnew;
     if (fabs(W) > BIG) return -103;
-    if (fabs((W - Wprev) / Wprev) < CONV && err < 1.e-1) break;
+    if (fabs((W - Wprev) / Wprev) < CONV && F.err < 1.e-1) break;
     if (!(iter < 50)) break;
+    F = Fn;
+    have = true;
   }
   return 0;
 }
@@ -655,9 +698,10 @@ __device__ inline int u2p_solver_W_warp(const Grid &G, const double *uu, double 
   U2PState s;
   u2p_setup(uu, g, s);
   double W = u2p_initial_w(G.gamma, pp, g);
-  if (u2p_bracket(G.gamma, Etype, s.c, W, fevals)) return -150;
+  U2PF F;
+  if (u2p_bracket(G.gamma, Etype, s.c, W, F, fevals)) return -150;
   int iter = 0;
-  int r = u2p_newton_warp(G.gamma, G.u2pconv, Etype, s.c, W, iter);
+  int r = u2p_newton_warp(G.gamma, G.u2pconv, Etype, s.c, W, iter, F, true);
   if (iters) *iters += (unsigned)iter;
   if (r < 0) return r;
   return u2p_final(G.gamma, s, W, iter, uu, pp, g);
@@ -709,9 +753,8 @@ KG_HD int u2p_solver_W(const Grid &G, const double *uu, double *pp, const Geom &
   U2PState s;
   u2p_setup(uu, g, s);
   double W = u2p_initial_w(G.gamma, pp, g);
-  if (u2p_bracket(G.gamma, Etype, s.c, W, fevals)) return -150;
   int iter = 0;
-  int r = u2p_newton(G.gamma, G.u2pconv, Etype, s.c, W, iter, 1 << 30, 1 << 30, fevals, fcap);
+  int r = u2p_solve_w(G.gamma, G.u2pconv, Etype, s.c, W, iter, 1 << 30, 1 << 30, fevals, fcap);
   if (r == U2P_OVER_CAP) return r;
   if (iters) *iters += (unsigned)iter;
   if (r < 0) return r;

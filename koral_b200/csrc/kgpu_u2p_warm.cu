@@ -63,9 +63,8 @@ __device__ int solve_from(const Grid &G, const double *uu, double *pp, const Geo
                           unsigned &iters, unsigned &fevals) {
   U2PState s;
   u2p_setup(uu, g, s);
-  if (u2p_bracket(G.gamma, Etype, s.c, W, &fevals)) return -150;
   int iter = 0;
-  const int r = u2p_newton(G.gamma, G.u2pconv, Etype, s.c, W, iter, 1 << 30, 1 << 30, &fevals, 0u);
+  const int r = u2p_solve_w(G.gamma, G.u2pconv, Etype, s.c, W, iter, 1 << 30, 1 << 30, &fevals, 0u);
   iters += (unsigned)iter;
   if (r < 0) return r;
   return u2p_final(G.gamma, s, W, iter, uu, pp, g);
