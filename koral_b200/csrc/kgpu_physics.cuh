@@ -690,11 +690,12 @@ __device__ inline int u2p_newton_warp(double GAMMA, double CONV, int Etype, cons
 
 #ifdef __CUDACC__
 KG_HD int u2p_final(double GAMMA, const struct U2PState &s, double W, int iter, const double *uu, double *pp,
-                    const Geom &g);
+                    const Geom &g, bool entropy);
 // u2p_solver_W with all 32 lanes of a warp on the same cell: the damped
 // trials of a Newton step are tried 32 at a time; same result.
 __device__ inline int u2p_solver_W_warp(const Grid &G, const double *uu, double *pp, const Geom &g, int Etype,
-                                        unsigned *iters = nullptr, unsigned *fevals = nullptr) {
+                                        unsigned *iters = nullptr, unsigned *fevals = nullptr,
+                                        bool entropy = true) {
   U2PState s;
   u2p_setup(uu, g, s);
   double W = u2p_initial_w(G.gamma, pp, g);
@@ -704,12 +705,15 @@ __device__ inline int u2p_solver_W_warp(const Grid &G, const double *uu, double 
   int r = u2p_newton_warp(G.gamma, G.u2pconv, Etype, s.c, W, iter, F, true);
   if (iters) *iters += (unsigned)iter;
   if (r < 0) return r;
-  return u2p_final(G.gamma, s, W, iter, uu, pp, g);
+  return u2p_final(G.gamma, s, W, iter, uu, pp, g, entropy);
 }
 #endif
 
-// checks and primitives from the converged W (u2p.c:2205-2292)
-KG_HD int u2p_final(double GAMMA, const U2PState &s, double W, int iter, const double *uu, double *pp, const Geom &g) {
+// checks and primitives from the converged W (u2p.c:2205-2292); entropy =
+// false leaves pp[5] alone, for a caller that needs no entropy yet and forms
+// it from the final density and energy (two powers and a logarithm)
+KG_HD int u2p_final(double GAMMA, const U2PState &s, double W, int iter, const double *uu, double *pp, const Geom &g,
+                    bool entropy = true) {
   if (iter >= 50) return -102;
   if (!isfinite(W)) return -103;
   const double gdetu = g.gdet;
@@ -732,7 +736,7 @@ KG_HD int u2p_final(double GAMMA, const U2PState &s, double W, int iter, const d
   pp[3] = ut2;
   pp[4] = ut3;
   if (rho < 0.) return -105;
-  pp[5] = calc_Sfromu(GAMMA, rho, uint);
+  if (entropy) pp[5] = calc_Sfromu(GAMMA, rho, uint);
   if (kMagn) {
     pp[B1] = uu[B1] / gdetu;
     pp[B2] = uu[B2] / gdetu;
@@ -749,7 +753,8 @@ KG_HD int u2p_final(double GAMMA, const U2PState &s, double W, int iter, const d
 // fcap the solve gives up (U2P_OVER_CAP, pp untouched) once *fevals reaches
 // fcap during the Newton steps
 KG_HD int u2p_solver_W(const Grid &G, const double *uu, double *pp, const Geom &g, int Etype,
-                       unsigned *iters = nullptr, unsigned *fevals = nullptr, unsigned fcap = 0) {
+                       unsigned *iters = nullptr, unsigned *fevals = nullptr, unsigned fcap = 0,
+                       bool entropy = true) {
   U2PState s;
   u2p_setup(uu, g, s);
   double W = u2p_initial_w(G.gamma, pp, g);
@@ -758,7 +763,7 @@ KG_HD int u2p_solver_W(const Grid &G, const double *uu, double *pp, const Geom &
   if (r == U2P_OVER_CAP) return r;
   if (iters) *iters += (unsigned)iter;
   if (r < 0) return r;
-  return u2p_final(G.gamma, s, W, iter, uu, pp, g);
+  return u2p_final(G.gamma, s, W, iter, uu, pp, g, entropy);
 }
 
 // high-level inversion with entropy fallback and "keep old" last resort

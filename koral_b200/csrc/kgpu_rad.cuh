@@ -406,10 +406,10 @@ KG_RAD_CALL KG_HD int imp_u2p_hot(const RadParams &R, const double *uu, double *
   G.nv = NVMAX;
   unsigned *st = inner ? inner->stats : nullptr;
 #ifdef __CUDA_ARCH__
-  if (inner && inner->warp) return u2p_solver_W_warp(G, uu, pp, g, 0, st, st ? st + 1 : nullptr);
+  if (inner && inner->warp) return u2p_solver_W_warp(G, uu, pp, g, 0, st, st ? st + 1 : nullptr, false);
 #endif
   unsigned used = 0;
-  const int r = u2p_solver_W(G, uu, pp, g, 0, st, &used, inner ? inner->cap : 0u);
+  const int r = u2p_solver_W(G, uu, pp, g, 0, st, &used, inner ? inner->cap : 0u, false);
   if (st) st[1] += used;
   return r;
 }
@@ -455,12 +455,16 @@ KG_HD void imp_rho_from_velocity(const double *uu0, double *pp, const Geom &g) {
 
 // The part of every evaluation that precedes the residual (rad.c:130-198,
 // 880-960): the density that follows the gas velocity when iterating MHD
-// primitives, the entropy, the conserved state that goes with pp, and the
-// inversion of the other component (which updates pp in place).
+// primitives, the conserved state that goes with pp, and the inversion of
+// the other component (which updates pp in place).  The reference forms the
+// entropy of the state here and again at the end of the gas inversion; it
+// enters no residual (the entropy equation's residual takes the conserved
+// entropy that imp_counterpart sets), so it is formed once, from the
+// solution, when the cascade ends (imp_advance): two powers and a logarithm,
+// twice, off every evaluation.
 KG_HD int imp_prepare(const RadParams &R, const ImpParams &P, const double *uu0, double *pp, double *uu,
                       const RadGeom &rg, int &corr, const ImpInner *inner = nullptr) {
   if (P.prim == IMP_MHD) imp_rho_from_velocity(uu0, pp, rg.g);
-  pp[ENTR] = rad_Sfromu(R, pp[RHO], pp[UU]);
   return imp_counterpart(R, P.prim, uu0, pp, uu, rg, corr, inner);
 }
 
@@ -839,6 +843,7 @@ KG_HD int imp_advance(const RadParams &R, const double *uu0, const double *pp00,
   for (int i = 0; i < NVR; i++) s.pp[i] = pin[i];
   if (P.prim == IMP_MHD && corr > 0) u2pret = -2;
   if (u2pret < -1) return imp_next_attempt(pp00, warm_guess, s, wa);
+  s.pp[ENTR] = rad_Sfromu(R, s.pp[RHO], s.pp[UU]);
   return IMP_DONE_OK;
 }
 
