@@ -364,7 +364,7 @@ int kgpu_rad_default_params(kgpu_rad_params *rp, double mass, double gamma, doub
 
 /* Solver variants of kgpu_rad_implicit_cells. */
 #define KGPU_RAD_PLAIN 0       /* one thread runs a cell's whole cascade        */
-#define KGPU_RAD_BATCHED 1     /* passes over a work queue of unfinished cells  */
+#define KGPU_RAD_BATCHED 1     /* four lanes a cell, cells from work lists      */
 #define KGPU_RAD_PERSISTENT 2  /* one resident kernel whose lanes take cells    */
                                /* from a work list as they finish, then a       */
                                /* warp-per-cell kernel for the cells left over  */
@@ -373,15 +373,15 @@ int kgpu_rad_default_params(kgpu_rad_params *rp, double mass, double gamma, doub
  * (Newton iterations, evaluations) do not depend on any field except
  * warm_attempts, which chooses how long a warm-started cell trusts its
  * prediction.
- *  pass_iters     batched: Newton iterations a cell may take per pass (4)
+ *  pass_iters     accepted and without effect (4): the batched form has no
+ *                 passes
  *  inner_cap      W-function evaluations the MHD inversion nested in one
- *                 residual evaluation may take in a single lane before that
- *                 evaluation is repeated by a whole warp with the damped
- *                 trials tried 32 at a time (64; 0: never)
- *  tail           batched: the size of the warp-per-cell tail, in blocks of
- *                 four warps per SM (0..32, default 8; 0: none): once the
- *                 cells left after a pass are no more than its warps, each is
- *                 run to its end by a whole warp
+ *                 residual evaluation may take in a single lane before a
+ *                 whole warp takes it, with the damped trials tried 32 at a
+ *                 time (64; 0: never).  The persistent form repeats the
+ *                 evaluation; the batched one goes on where the lane stopped,
+ *                 and does so after a quarter of them
+ *  tail           accepted and without effect (0..32, default 8)
  *  warm_attempts  learned warm start: attempts of the cascade a warm-started
  *                 cell runs from the predicted iterate before the reference
  *                 cascade runs from the reference guess (1..6, default 6)
@@ -398,13 +398,7 @@ int kgpu_rad_default_params(kgpu_rad_params *rp, double mass, double gamma, doub
  *                 prediction, the others from their own guess; 0: every
  *                 warm-started cell begins with attempt 0.  Every cell still
  *                 converges to RADIMPCONV or runs the reference cascade
- *  hard           batched, in a context's implicit step: a cell whose
- *                 previous solve in that context took a later attempt,
- *                 failed, or took more than `hard` Newton iterations skips
- *                 the first pass and starts in the warp-per-cell tail, where
- *                 long cascades run fastest (default 16; -1: every cell
- *                 starts in the first pass; the context-free entry points
- *                 have no previous solve and ignore it) */
+ *  hard           accepted and without effect (-1.., default 16) */
 typedef struct {
   int pass_iters;
   int inner_cap;
@@ -627,9 +621,8 @@ int kgpu_set_tuning(kgpu_ctx *ctx, const kgpu_tuning *t);
  * times them with CUDA events; the state, the time step and the counters
  * are restored afterwards, and the choice is applied.  Candidates: the
  * fused or split face flux, flux 5..8, update 3..5, u2p 4..6 blocks; u2p_pass_iters 4, 8, 16; with
- * radiation the batched and the persistent solver, pass_iters 4, 8, 16,
- * inner_cap 32, 64, 128, tail 0, 4, 8, 16, hard -1, 8, 16, 32 or thin 4, 8,
- * 16.  A candidate
+ * radiation the batched and the persistent solver, inner_cap 32, 64, 128 and,
+ * persistent, thin 4, 8, 16.  A candidate
  * replaces the incumbent only when it is faster by min_gain (a fraction,
  * e.g. 0.02) in the same round of trials.  The choice is cached per device
  * and grid configuration for the process: with reuse = 1 a cached choice

@@ -30,6 +30,15 @@
 
 namespace kgpu {
 
+// the library's pow, one copy of it for every caller: its special cases are
+// as long as the function, and the implicit solve is bound by the fetch of
+// its instructions
+#if defined(__CUDACC__)
+static __host__ __device__ __noinline__ double pow_call(double x, double y) { return pow(x, y); }
+#else
+static double pow_call(double x, double y) { return pow(x, y); }
+#endif
+
 // double-double number hi + lo, |lo| <= ulp(hi)/2
 struct DD {
   double hi, lo;
@@ -92,7 +101,7 @@ KM_HD bool pw_in_range(double x, double y) {
 
 // x^4 = (x^2)^2 with x^2 kept exact as a double-double
 KM_HD double pw4(double x) {
-  if (!pw_in_range(fabs(x), 4.)) return pow(x, 4.);
+  if (!pw_in_range(fabs(x), 4.)) return pow_call(x, 4.);
   const DD t = dd_two_prod(x, x);
   const DD q = dd_mul(t, t);
   return q.hi + q.lo;

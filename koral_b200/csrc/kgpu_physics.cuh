@@ -512,8 +512,9 @@ KG_HD double u2p_initial_w(double GAMMA, const double *pp, const Geom &g) {
 }
 
 constexpr int U2P_PAUSED = 1;
-// returned by a capped W solve that used up its function evaluations (the
-// caller repeats the whole inversion another way; nothing is kept)
+// returned by a capped W solve that used up its function evaluations, (W,
+// iter) as at the start of the running iteration: u2p_newton_warp may go on
+// from there, or the caller repeats the inversion another way
 constexpr int U2P_OVER_CAP = 7;
 
 // The W function at one point.
@@ -561,7 +562,10 @@ KG_HD int u2p_solve_w(double GAMMA, double CONV, int Etype, const U2PCons &c, do
         if (n >= 50) return -150;
       } else {
         if (bad && n < 100) {
-          if (fcap && *fevals >= fcap) return U2P_OVER_CAP;
+          if (fcap && *fevals >= fcap) {
+            iter--;
+            return U2P_OVER_CAP;
+          }
           n++;
           if (n >= damp_budget) {
             iter--;
@@ -635,56 +639,57 @@ __device__ inline int u2p_newton_warp(double GAMMA, double CONV, int Etype, cons
                                       U2PF F = U2PF{0., 0., 0.}, bool have = false) {
   const int lane = threadIdx.x & 31;
   const double D = c.D;
-  while (true) {
-    double Wprev = W;
+  U2PF S{0., 0., 0.};      // the function where the running step started
+  int base = -1;           // first of the 32 halvings tried; -1: the evaluation is at W itself
+  if (have) {
+    S = F;
     iter++;
-    if (!have) f_u2p(GAMMA, Etype, W - D, c, F.f, F.df, F.err);
-    have = false;
-    if (F.err < CONV) break;
-    if (F.df == 0.) {
-      W *= 1.1;
-      if (iter < 50) continue;
-      break;
-    }
-    double Wnew = 0.;
-    U2PF Fn = F;
-    int found = -1;
-    for (int base = 0; base <= 100 && found < 0; base += 32) {
-      const int k = base + lane;
-      double Wk = 0.;
-      U2PF T{0., 0., 0.};
-      bool accept = false;
-      if (k == 0) {
-        Wk = W - F.f / F.df;
-      } else if (k <= 100) {
-        const double dumpfac = ldexp(1.0, -k);
-        Wk = W - dumpfac * F.f / F.df;
-      }
-      if (k == 100) {
-        accept = true;   // the scalar loop stops here whatever the state
-      } else if (k < 100) {
-        f_u2p(GAMMA, Etype, Wk - D, c, T.f, T.df, T.err);
-        accept = !u2p_bad_w(Wk, c.Bsq, c.QdotBsq, c.Qt2, T.f, T.df);
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, accept);
-      if (m) {
-        const int L = __ffs(m) - 1;
-        found = base + L;
-        Wnew = __shfl_sync(0xffffffffu, Wk, L);
-        Fn.f = __shfl_sync(0xffffffffu, T.f, L);
-        Fn.df = __shfl_sync(0xffffffffu, T.df, L);
-        Fn.err = __shfl_sync(0xffffffffu, T.err, L);
-      }
-    }
-    if (found >= 100) return -101;
-    W = Wnew;
-    if (fabs(W) > BIG) return -103;
-    if (fabs((W - Wprev) / Wprev) < CONV && F.err < 1.e-1) break;
-    if (!(iter < 50)) break;
-    F = Fn;
-    have = true;
+    if (S.err < CONV) return 0;
+    base = 0;
   }
-  return 0;
+  while (true) {
+    // one evaluation by every lane: at W, or at halving k of the running step
+    const int k = base + lane;
+    double at = W;
+    if (base >= 0) {
+      if (S.df == 0.) {
+        W *= 1.1;
+        if (!(iter < 50)) return 0;
+        base = -1;
+        continue;
+      }
+      at = k == 0 ? W - S.f / S.df : W - ldexp(1.0, -(k < 100 ? k : 100)) * S.f / S.df;
+    }
+    U2PF T;
+    f_u2p(GAMMA, Etype, at - D, c, T.f, T.df, T.err);
+    if (base < 0) {
+      S = T;
+      iter++;
+      if (S.err < CONV) return 0;
+      base = 0;
+      continue;
+    }
+    // the scalar loop stops at halving 100 whatever the state
+    const bool accept = k == 100 || (k < 100 && !u2p_bad_w(at, c.Bsq, c.QdotBsq, c.Qt2, T.f, T.df));
+    const unsigned m = __ballot_sync(0xffffffffu, accept);
+    if (!m) {
+      base += 32;
+      continue;
+    }
+    const int L = __ffs(m) - 1;
+    if (base + L >= 100) return -101;
+    const double Wprev = W, err = S.err;
+    W = __shfl_sync(0xffffffffu, at, L);
+    S.f = __shfl_sync(0xffffffffu, T.f, L);
+    S.df = __shfl_sync(0xffffffffu, T.df, L);
+    S.err = __shfl_sync(0xffffffffu, T.err, L);
+    if (fabs(W) > BIG) return -103;
+    if (fabs((W - Wprev) / Wprev) < CONV && err < 1.e-1) return 0;
+    if (!(iter < 50)) return 0;
+    iter++;
+    if (S.err < CONV) return 0;
+    base = 0;
+  }
 }
 #endif
 

@@ -1,26 +1,21 @@
 // Batched implicit gas-radiation source solve and M1 closure on the GPU.
 //
-// Two forms of the per-cell cascade of solve_implicit_lab (rad.c:1225):
+// Three forms of the per-cell cascade of solve_implicit_lab (rad.c:1225):
 //  - plain: one thread runs a cell's cascade from the first attempt to the
 //    last; a warp takes as long as its slowest cell;
-//  - batched: passes over a work queue.  A pass gives every unfinished cell
-//    a budget of Newton iterations; a cell whose attempt fails goes on with
-//    the next attempt inside the same budget; a cell that runs out of budget
-//    keeps its iterate and iteration count (the whole loop-carried state of
-//    the Newton solve) and is appended to the next pass's queue.  Cells
-//    that finish leave the queue, so warps stay full of live work.  The
-//    iterations a cell takes are the same in both forms (the solve resumes
-//    exactly where it stopped), so both give the same results.
+//  - batched: one resident kernel (k_rad_quads) in which four lanes work on a
+//    cell and take the next one of a work list as soon as theirs is done;
 //  - persistent: one resident kernel (k_rad_persist) whose lanes take cells
 //    from a work list and take the next one as soon as theirs finishes, so
 //    no lane waits for a pass to end; cells whose nested inversion runs
 //    over its cap, and those still running in warps that have thinned out
 //    once the list is empty, are handed with their whole state to a
 //    warp-per-cell kernel (k_rad_finish) that runs them to their end.  Three
-//    launches per solve instead of one per pass; the same bits.
-// Both run the cascade as the one-evaluation state machine of
-// kgpu_rad.cuh (imp_advance), so the lanes of a warp perform their
-// expensive evaluations together whatever phase each cell is in.
+//    launches per solve; the same bits.
+// Plain and persistent run the cascade as the one-evaluation state machine
+// of kgpu_rad.cuh (imp_advance), so the lanes of a warp perform their
+// expensive evaluations together whatever phase each cell is in; the batched
+// form runs the same evaluations and transitions for four lanes a cell.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -39,10 +34,7 @@ using namespace kgpu;
 #ifndef KGPU_RAD_MIN_BLOCKS
 #define KGPU_RAD_MIN_BLOCKS 4
 #endif
-// default size of the warp-per-cell tail, in blocks of four warps per SM
-// (kgpu_rad_solver_opts.tail): 8 = two waves at 4 resident blocks; measured
-// on the same steps with 4 Newton iterations per pass: 193.5 ms per step at
-// 4 blocks, 189.1 at 6, 187.3 at 8
+// default of kgpu_rad_solver_opts.tail
 #ifndef KGPU_RAD_TAIL_BLOCKS
 #define KGPU_RAD_TAIL_BLOCKS 8
 #endif
@@ -76,16 +68,14 @@ RadParams to_dev(const kgpu_rad_params &p) {
 
 // Tuning of the batched and persistent forms (kgpu_rad_solver_opts)
 struct Opts {
-  int pass_iters = 4;       // Newton iterations per cell and pass of the batched form (4: 1674 against
-                            // 1743 ms at 8 on 2^21 batched-solve cells, 77.7 against 81.7 ms on a
-                            // settled torus solve)
+  int pass_iters = 4;       // kept for callers that set it: the batched form has no passes any more
   int inner_cap = 64;       // W-function evaluations of a nested inversion in one lane (0: no cap)
-  int tail = KGPU_RAD_TAIL_BLOCKS;   // batched: blocks per SM of the warp-per-cell tail (0: none)
+  int tail = KGPU_RAD_TAIL_BLOCKS;   // kept likewise (it sized a tail of the passes)
   int warm_attempts = IMP_NATTEMPTS;
   int thin = 8;             // persistent: hand-off threshold of live lanes once the list is empty
   int blocks_per_sm = 0;    // persistent: resident blocks per SM (0: occupancy limit)
   int skip = 1;             // warm start: begin with the attempt the network expects to succeed
-  int hard = 16;            // batched, context: cells hard in their previous solve start in the tail (-1: off)
+  int hard = 16;            // kept likewise (it routed cells to that tail)
 };
 Opts g_opts;   // the context-free entry points' values
 
@@ -119,14 +109,10 @@ bool opts_valid(const kgpu_rad_solver_opts &o) {
          o.blocks_per_sm <= 16 && o.skip >= 0 && o.skip <= 2 && o.hard >= -1;
 }
 
-// upper bound of the passes a cell can need: six attempts of at most
-// RADIMPMAXITER + 1 iterations each (the queue-length array of the work
-// area has room for kMaxPasses)
-constexpr int kMaxPasses = 4096;
-int max_passes(const RadParams &R, int K) {
-  int p = (int)((IMP_NATTEMPTS * (R.maxiter + 1) + K - 1) / K) + 1;
-  return p < kMaxPasses ? p : kMaxPasses;
-}
+// counters of the work area: [0..3] list lengths at the start, [8..11]
+// entries to take, [16..19] next places, [24..27] places reserved, [64..] what
+// each SM is at
+constexpr int kCounters = 64 + 1024;
 
 struct Cell {
   const double *uu, *pp, *g, *G, *dt;
@@ -142,8 +128,8 @@ struct Work {
   int *wsw;         // [n] which primitives the cascade starts with
   int *wwarm;       // [n] the cascade still runs from the predicted iterate
   double *wguess;   // [n][13] the predicted iterate (warm start only)
-  int *q[2][2];     // queues of cell indices [pass parity][primitives of the running attempt]
-  int *count;       // [passes + 2][3] queue lengths: the two queues of a pass, then its cooperative queue
+  int *q[2][2];     // queues of cell indices (persistent form)
+  int *count;       // [kCounters]
   int *qs;          // cooperative queue of the current pass: cell indices ...
   ImpState *ss;     // ... and the states of their interrupted evaluations
   int nslots;       // its capacity
@@ -161,7 +147,7 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // finds the queue full carries on alone, without the cap)
 inline int slow_slots(int n) { return n / 8 > 1024 ? n / 8 : 1024; }
 
-size_t work_layout(int n, int passes, Work *w, char *base) {
+size_t work_layout(int n, Work *w, char *base) {
   size_t off = 0;
   auto take = [&](size_t bytes) {
     size_t o = off;
@@ -180,7 +166,7 @@ size_t work_layout(int n, int passes, Work *w, char *base) {
       p = take((size_t)n * 4);
       if (w) w->q[a][b] = (int *)p;
     }
-  p = take((size_t)(passes + 2) * 3 * 4); if (w) w->count = (int *)p;
+  p = take((size_t)kCounters * 4); if (w) w->count = (int *)p;
   p = take(8 * sizeof(unsigned long long)); if (w) w->stats = (unsigned long long *)p;
   p = take(sizeof(unsigned)); if (w) w->tail_done = (unsigned *)p;
   p = take(4 * sizeof(unsigned)); if (w) w->ctl = (unsigned *)p;
@@ -260,75 +246,54 @@ __global__ void __launch_bounds__(128, KGPU_RAD_MIN_BLOCKS) k_rad_plain(RadParam
   }
 }
 
-// Start of the batched form: every cell's cascade state (first attempt,
-// no iteration yet, the guess as iterate), queued by the primitives its
-// first attempt works on, so that warps of a pass run one kind of inversion.
-// gate >= 0: only cells whose previous solve (the attempt and iteration
-// outputs, read before this solve overwrites them) needed a later attempt
-// or more than gate Newton iterations start from the prediction
-// skip 1: a warm-started cell begins with the attempt the network expects
-// to be the first that succeeds (mlp_first_attempt) instead of the first
-// one; skip 2: besides, only the cells the network expects to fail their
-// first attempt start from the prediction, the others from their own guess
-// hard >= 0 (batched form, where attempt and iteration outputs of a
-// previous solve are valid): a cell whose previous solve took a later
-// attempt, failed, or took more than `hard` iterations goes to the queue of
-// the second pass instead of the first, so that the warp-per-cell tail,
-// which follows the first pass, starts it; the cell's arithmetic is the same
-// in either kernel
-// Cells whose previous solve was hard (the routing test of k_rad_start),
-// counted into *count.
-__global__ void k_rad_count_hard(Cell C, int n, int hard, unsigned *count) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool late = k < n && (C.attempt[k] != 0 || C.iters[k] > hard);
-  const unsigned m = __ballot_sync(0xffffffffu, late);
-  if ((threadIdx.x & 31) == 0 && m) atomicAdd(count, (unsigned)__popc(m));
-}
+// Work lists, one per kind of attempt (frame and primitives).  An entry is a
+// cell with its running attempt, whether its cascade is warm-started, and
+// the primitives it starts with, in one 64-bit word (0: not written yet).
+// `avail` counts the entries that may be taken, `next` and `tail` the places
+// taken and reserved.
+struct QuadList {
+  unsigned long long *e;
+  int *avail, *next, *tail;
+};
+struct QuadLists {
+  QuadList l[4];   // [frame * 2 + primitives]
+};
+constexpr int QUAD_LAB_TURNS = 4, QUAD_FF_TURNS = 2;   // times a cell can enter a list of either frame
 
-__global__ void k_rad_start(RadParams R, Cell C, Work W, int n, const float *ypred, int gate, int skip, int hard,
-                            int limit) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  RadGeom rg;
-  rad_geom(C.g + 20L * k, C.G + 20L * k, rg);
-  const double *p0 = C.pp + (long)k * NVR;
-  const int sw = imp_startwith(R, p0, rg.g);
-  int first = 0;
-  W.wsw[k] = sw;
-  W.wit[k] = 0;
-  double t[MLP_OUT];
-  bool warm = ypred && (gate < 0 || C.attempt[k] != 0 || C.iters[k] > gate);
-  if (warm) {
-    for (int o = 0; o < MLP_OUT; o++) t[o] = ypred[(long)k * MLP_OUTP + o];
-    if (skip == 2 && mlp_first_attempt(t) == 0) warm = false;
-  }
-  if (warm) {
-    // learned warm start: the first attempt begins at the predicted state
-    double guess[NVR];
-    mlp_guess(p0, rg, sw, t, guess);
-    if (skip) first = mlp_first_attempt(t);
-    for (int i = 0; i < NVR; i++) {
-      W.wpp[(long)k * NVR + i] = guess[i];
-      W.wguess[(long)k * NVR + i] = guess[i];
+__device__ inline unsigned long long quad_entry(int k, int att, int warm, int sw) {
+  return (unsigned long long)(unsigned)k | ((unsigned long long)(unsigned)(256 | sw << 4 | warm << 3 | att) << 32);
+}
+// appends a cell; called by one lane
+__device__ inline void quad_push(const QuadList &L, unsigned long long e) {
+  *(volatile unsigned long long *)(L.e + atomicAdd(L.tail, 1)) = e;
+  __threadfence();
+  atomicAdd(L.avail, 1);
+}
+// takes up to `want` entries; called by one lane.  A taker that finds too
+// few gives back what it could not have, and looks again if what is left is
+// then positive (another's push or return met its own), so an entry is never
+// left behind by the last one to look.
+__device__ inline int quad_take(const QuadList &L, int want, int &at) {
+  while (true) {
+    if (*(volatile int *)L.avail <= 0) return 0;
+    const int had = atomicSub(L.avail, want);
+    const int got = had >= want ? want : (had > 0 ? had : 0);
+    int left = 0;
+    if (got < want) left = atomicAdd(L.avail, want - got) + want - got;
+    if (got > 0) {
+      at = atomicAdd(L.next, got);
+      return got;
     }
-    W.wwarm[k] = 1;
-  } else {
-    for (int i = 0; i < NVR; i++) W.wpp[(long)k * NVR + i] = p0[i];
-    W.wwarm[k] = 0;
+    if (left <= 0) return 0;
   }
-  W.watt[k] = first;
-  // the queue is chosen by the predicate, never by the pointer: every lane
-  // of a warp-aggregated push must name the same queue
-  const int type = imp_attempt(first, sw).prim;
-  // the routing applies only when all such cells fit in the tail (limit
-  // warps); with more of them (the transient of a run) every cell starts in
-  // the first pass.  The count is read from device memory, the same value
-  // in every block
-  const bool late = hard >= 0 && W.ctl[0] <= (unsigned)limit && (C.attempt[k] != 0 || C.iters[k] > hard);
-  warp_push(W.q[0][0], W.count + 0, !late && type == 0, k);
-  warp_push(W.q[0][1], W.count + 1, !late && type == 1, k);
-  warp_push(W.q[1][0], W.count + 3, late && type == 0, k);
-  warp_push(W.q[1][1], W.count + 4, late && type == 1, k);
+}
+// an entry taken: its writer is between reserving the place and writing it
+// at most, so the wait is short; it is bounded all the same (a cell given up
+// keeps the failure status it starts with)
+__device__ inline unsigned long long quad_read(const QuadList &L, int at) {
+  unsigned long long e = 0;
+  for (int i = 0; i < 1 << 20 && e == 0; i++) e = *(volatile unsigned long long *)(L.e + at);
+  return e;
 }
 
 // warp-aggregated append that returns each pushing lane's slot (or -1)
@@ -343,216 +308,597 @@ __device__ inline int warp_slot(int *qcount, bool pred) {
   return pred ? base + __popc(bits & ((1u << lane) - 1u)) : -1;
 }
 
-// Pass p: the cells of queue p may start up to K Newton iterations;
-// unfinished ones keep their state (the iterate, its iteration count, the
-// attempt) and go to queue p+1, by the primitives of their running attempt.
-__global__ void __launch_bounds__(128, KGPU_RAD_MIN_BLOCKS) k_rad_pass(RadParams R, Cell C, Work W, int n, int p, int K,
-                                                  unsigned inner_cap, int warm_attempts) {
-  const int n0 = W.count[p * 3 + 0], n1 = W.count[p * 3 + 1];
-  const int nin = n0 + n1;
-  const int par = p & 1;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nin; q += gridDim.x * blockDim.x) {
-    const int k = q < n0 ? W.q[par][0][q] : W.q[par][1][q - n0];
-    RadGeom rg;
-    rad_geom(C.g + 20L * k, C.G + 20L * k, rg);
-    const double *u0 = C.uu + (long)k * NVR, *p0 = C.pp + (long)k * NVR;
-    const double dt = C.dt[k];
-    ImpState s;
-    s.phase = PH_BASE;
-    s.j = 0;
-    s.sign = -1.;
-    s.xiapp = 1.;
-    s.evals = 0;
-    s.inner[0] = s.inner[1] = 0;
-    s.sw = W.wsw[k];
-    s.att = W.watt[k];
-    s.iter = W.wit[k];
-    s.warm = W.wwarm[k];
-    for (int i = 0; i < NVR; i++) s.pp[i] = W.wpp[(long)k * NVR + i];
-    const int warm0 = s.warm;
-    int budget = K;
-    int r;
-    const double *wg = W.wguess + (long)k * NVR;
-    ImpInner how{nullptr, inner_cap, false, warm_attempts};
-    while (true) {
-      while ((r = imp_advance(R, u0, p0, dt, rg, s, budget, wg, &how)) == IMP_RUNNING) {
-      }
-      // an evaluation whose nested inversion ran out of its cap goes to the
-      // cooperative pass with the whole state; with the queue full the lane
-      // repeats it alone, without the cap
-      const int slot = warp_slot(W.count + p * 3 + 2, r == IMP_OVER_CAP);
-      if (r != IMP_OVER_CAP) break;
-      if (slot < W.nslots) {
-        W.qs[slot] = k;
-        W.ss[slot] = s;
-        break;
-      }
-      how.cap = 0;
+// Start of the batched form: every cell's cascade state (first attempt,
+// no iteration yet, the guess as iterate), queued by the primitives its
+// first attempt works on, so that warps of a pass run one kind of inversion.
+// gate >= 0: only cells whose previous solve (the attempt and iteration
+// outputs, read before this solve overwrites them) needed a later attempt
+// or more than gate Newton iterations start from the prediction
+// skip 1: a warm-started cell begins with the attempt the network expects
+// to be the first that succeeds (mlp_first_attempt) instead of the first
+// one; skip 2: besides, only the cells the network expects to fail their
+// first attempt start from the prediction, the others from their own guess
+// keep: the iterate goes to the work area too (the persistent form, which
+// resumes cells from it)
+__global__ void k_rad_start(RadParams R, Cell C, Work W, QuadLists Q, int n, const float *ypred, int gate, int skip,
+                            bool keep) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  RadGeom rg;
+  rad_geom(C.g + 20L * k, C.G + 20L * k, rg);
+  const double *p0 = C.pp + (long)k * NVR;
+  const int sw = imp_startwith(R, p0, rg.g);
+  int first = 0;
+  if (keep) {
+    W.wsw[k] = sw;
+    W.wit[k] = 0;
+  }
+  double t[MLP_OUT];
+  bool warm = ypred && (gate < 0 || C.attempt[k] != 0 || C.iters[k] > gate);
+  if (warm) {
+    for (int o = 0; o < MLP_OUT; o++) t[o] = ypred[(long)k * MLP_OUTP + o];
+    if (skip == 2 && mlp_first_attempt(t) == 0) warm = false;
+  }
+  if (warm) {
+    // learned warm start: the first attempt begins at the predicted state
+    double guess[NVR];
+    mlp_guess(p0, rg, sw, t, guess);
+    if (skip) first = mlp_first_attempt(t);
+    for (int i = 0; i < NVR; i++) {
+      if (keep) W.wpp[(long)k * NVR + i] = guess[i];
+      W.wguess[(long)k * NVR + i] = guess[i];
     }
-    warp_add(W.stats, (unsigned)(K - budget));
-    warp_add(W.stats + 2, (unsigned)(warm0 && !s.warm));
-    warp_add(W.stats + 3, s.evals);
-    warp_add(W.stats + 4, s.inner[0]);
-    warp_add(W.stats + 5, s.inner[1]);
-    warp_add(W.stats + 6, (unsigned)(r == IMP_OVER_CAP));
-    if (r == IMP_OVER_CAP) continue;
-    const bool paused = r == IMP_PAUSE;
-    const int type = paused ? imp_attempt(s.att, s.sw).prim : 0;
-    warp_push(W.q[par ^ 1][0], W.count + (p + 1) * 3 + 0, paused && type == 0, k);
-    warp_push(W.q[par ^ 1][1], W.count + (p + 1) * 3 + 1, paused && type == 1, k);
-    if (paused) {
-      W.watt[k] = s.att;
-      W.wit[k] = s.iter;
-      W.wwarm[k] = s.warm;
-      for (int i = 0; i < NVR; i++) W.wpp[(long)k * NVR + i] = s.pp[i];
-    } else if (r == IMP_DONE_OK) {
-      cell_success(R, C, k, rg, s.pp, s.att, s.iter);
+    if (keep) W.wwarm[k] = 1;
+  } else {
+    if (keep) {
+      for (int i = 0; i < NVR; i++) W.wpp[(long)k * NVR + i] = p0[i];
+      W.wwarm[k] = 0;
+    }
+  }
+  if (keep) W.watt[k] = first;
+  // the queue is chosen by the predicate, never by the pointer: every lane
+  // of a warp-aggregated push must name the same queue
+  const ImpParams P = imp_attempt(first, sw);
+  if (keep) {   // one list per primitives
+    warp_push(W.q[0][0], W.count + 0, P.prim == 0, k);
+    warp_push(W.q[0][1], W.count + 1, P.prim == 1, k);
+    return;
+  }
+  C.status[k] = -1;
+  const unsigned long long e = quad_entry(k, first, warm ? 1 : 0, sw);
+  for (int i = 0; i < (ypred ? 4 : 2); i++) {   // an attempt other than the first only from a prediction
+    const bool mine = P.frame * 2 + P.prim == i;
+    const int at = warp_slot(Q.l[i].tail, mine);
+    if (mine) Q.l[i].e[at] = e;
+  }
+}
+
+// The lists' counters as the resident kernel finds them: all of it there to
+// be taken.
+__global__ void k_rad_lists(QuadLists Q, int *start) {
+  const int i = threadIdx.x;
+  if (i < 4) start[i] = *Q.l[i].avail = *Q.l[i].tail;
+}
+
+// ---------------------------------------------------------------------------
+// The batched form: four lanes per cell.
+// ---------------------------------------------------------------------------
+// A Newton iteration is a base evaluation, four Jacobian columns and one or
+// more damped trials.  The columns do not depend on one another, so a group
+// of four lanes (a quad) works on a cell: in a Jacobian trip each lane
+// evaluates its own column, in the others the four do the same.  An
+// iteration is then two trips on MHD primitives (the base evaluation is the
+// accepted trial's, see imp_advance) and three on radiation primitives,
+// against five and six evaluations of one lane, for 8 and 12 lane
+// evaluations against 5 and 6.  What that buys: a solve is a chain of up to
+// a few hundred iterations in its longest cells, and everything but the
+// first few iterations of a batch is bound by that chain and by warps that
+// wait for their slowest lane (8 cells a warp wait for one another, not 32).
+//
+// What all lanes of a quad read (the metric, the cell's conserved state and
+// guess, the iterate, the Jacobian) lies in shared memory, 936 bytes a cell
+// (an odd number of doubles: the eight cells of a warp fall on different
+// banks), which leaves the registers to the evaluation.
+//
+// The code of a warp is specialised for the kind of attempt its cells are
+// running (the primitives iterated and the frame).  A cell stays with its
+// quad while its attempts are of one kind and otherwise goes to the list of
+// the next kind; a quad takes the next cell of its list as soon as its own is
+// done, so no lane waits for a pass to end.
+constexpr int QUAD_CELLS = 8;   // cells per warp
+constexpr int QUAD_WARPS = 8;   // warps per block
+constexpr int QUAD_BLOCKS = 2;  // blocks per SM: 16 warps of 128 registers
+struct QuadCell {
+  RadGeom rg;
+  double uu0[NVR], pp00[NVR];   // conserved state, guess
+  double pp[NVR], ppp[NVR];     // iterate, and the iterate at the start of the iteration
+  double J[4][4];               // Jacobian; its inverse once complete
+  double f1[4];                 // residual at ppp
+  double dt, Ehat0;
+};
+static_assert(sizeof(QuadCell) == 117 * sizeof(double), "an odd number of doubles, for the banks");
+
+// a value of v[i], i < 4, without indexing the registers
+__device__ inline double pick4(const double *v, int i) { return i == 0 ? v[0] : (i == 1 ? v[1] : (i == 2 ? v[2] : v[3])); }
+
+template <int PRIM, int FRAME>
+__device__ __forceinline__ void quads_run(const RadParams &R, const Cell &C, const Work &W, const QuadLists &Q,
+                                          QuadCell *cells, int ncells, bool lock, unsigned cap, int warm_attempts,
+                                          unsigned *st) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int sh = PRIM == IMP_MHD ? UU : EE0;
+  const int lane = threadIdx.x & 31, quad = lane >> 2, col = lane & 3;
+  QuadCell &q = cells[quad];
+  const QuadList &list = Q.l[FRAME * 2 + PRIM];
+  const auto together = [lock]() {
+    if (lock) __syncthreads();
+    else __syncwarp();
+  };
+  const bool idle = quad >= ncells;   // this warp takes fewer cells than it could
+  bool have = false;
+  int look = 0;                       // trips until an empty list is looked at again
+  // the running cell, the same in the four lanes of the quad
+  int k = 0, phase = PH_BASE, iter = 0, att = 0, sw = 0, warm = 0;
+  double xiapp = 1.;
+  bool careful = false;   // damped trials one by one (below)
+  // this lane's column of the running Jacobian
+  bool todo = false, minus = true;
+  unsigned cin0 = 0, cin1 = 0;
+  bool begin = false;   // the attempt starts with the next trip
+  while (true) {
+    // quads without a cell take the next ones of the list
+    const unsigned need = look-- > 0 ? 0u : __ballot_sync(FULL, col == 0 && !have && !idle);
+    if (need) {
+      const int leader = __ffs(need) - 1;
+      int base = 0, got = 0;
+      if (lane == leader) got = quad_take(list, __popc(need), base);
+      base = __shfl_sync(FULL, base, leader);
+      got = __shfl_sync(FULL, got, leader);
+      if (got < __popc(need)) look = 8;
+      if (!have && !idle) {
+        const int at = __popc(need & ((1u << (quad * 4)) - 1u));
+        unsigned long long e = 0;
+        if (at < got && col == 0) e = quad_read(list, base + at);
+        e = __shfl_sync(0xfu << (quad * 4), e, 0, 4);
+        if (e) {
+          k = (int)(unsigned)e;
+          const double *g = C.g + 20L * k, *G = C.G + 20L * k;
+          double *gg = &q.rg.g.gg[0][0], *GG = &q.rg.g.GG[0][0];
+#pragma unroll 1
+          for (int i = col; i < 20; i += 4) {
+            gg[i] = g[i];
+            GG[i] = G[i];
+          }
+#pragma unroll 1
+          for (int i = col; i < NVR; i += 4) {
+            q.uu0[i] = C.uu[(long)k * NVR + i];
+            q.pp00[i] = C.pp[(long)k * NVR + i];
+          }
+          if (col == 0) {
+            q.dt = C.dt[k];
+            q.rg.g.gdet = g[19];
+            q.rg.g.gttpert = G[19];
+            q.rg.alpha = sqrt(-1. / G[0]);
+          }
+          const int how = (int)(e >> 32);
+          att = how & 7;
+          warm = (how >> 3) & 1;
+          sw = (how >> 4) & 1;
+          have = begin = true;
+        }
+      }
+    }
+    if (!(lock ? __syncthreads_or(have) : __any_sync(FULL, have))) break;
+    __syncwarp();
+    const RadGeom &rg = q.rg;
+    if (begin) {
+      // an attempt starts from the guess, or from the predicted iterate
+      const double *src = warm ? W.wguess + (long)k * NVR : q.pp00;
+#pragma unroll 1
+      for (int i = col; i < NVR; i += 4) q.pp[i] = src[i];
+      if (PRIM == IMP_RAD && FRAME == IMP_FF && col == 0) q.Ehat0 = imp_Ehat(q.pp00, rg.g);
+      iter = 0;
+      phase = PH_BASE;
+      begin = false;
+    }
+    __syncwarp();
+    // the entropy equation is never solved in the fluid frame
+    const ImpParams P{PRIM, FRAME == IMP_FF ? (int)IMP_ENERGY : imp_attempt(att, sw).eq, FRAME};
+    // the input of this trip's evaluation
+    bool act = have && (phase != PH_JAC || todo);
+    int rejected = 0;   // trials of this trip that are not evaluated
+    double pin[NVR], uu[NVR], x[4] = {0., 0., 0., 0.};
+    {
+      const double *from = phase == PH_JAC ? q.ppp : q.pp;
+#pragma unroll
+      for (int i = 0; i < NVR; i++) pin[i] = from[i];
+    }
+    if (phase == PH_BASE) {
+      iter++;
+    } else if (phase == PH_JAC) {
+      const double del = imp_fd_step(R, col, minus ? -1. : 1., q.ppp[col + sh], rg.g);
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (i == col) pin[i + sh] = pin[i + sh] + del;
     } else {
-      cell_failure(C, k);
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0 && nin > 0) atomicAdd(W.stats + 1, 1ull);
-}
-
-// The tail of the batched form.  Launched after pass p (and its cooperative
-// part): when the cells those left unfinished are no more than its warps
-// (at most `limit`), each is taken by a whole warp and run to its end.  At
-// the start of every Newton iteration lanes 0..8 evaluate the base and the
-// four Jacobian columns on both sides together (imp_eval_entry), and the
-// state machine, run by every lane alike, takes those entries instead of
-// evaluating them one after another (ImpCache); damped trials and the final
-// inversion it evaluates itself, with warp-wide nested inversions.  The sequence of operations per cell, and
-// so its results and its statistics, are those of the passes; a cell's
-// latency falls from six evaluations per Newton iteration to about two.
-// The last block to finish empties the queue, so that the passes after
-// this one find no work.
-constexpr int TAIL_WARPS = 4;   // warps per block of 128
-__global__ void __launch_bounds__(128, KGPU_RAD_MIN_BLOCKS) k_rad_tail(RadParams R, Cell C, Work W, int n, int p, int limit,
-                                                  int warm_attempts) {
-  const int nq = p + 1;
-  const int n0 = W.count[nq * 3 + 0], n1 = W.count[nq * 3 + 1];
-  const int nin = n0 + n1;
-  if (nin == 0 || nin > limit) return;   // the same decision in every block
-  __shared__ ImpEval cache_sh[TAIL_WARPS][IMP_NCACHE];
-  const int par = nq & 1;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  ImpEval *ce = cache_sh[wib];
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < nin; q += nwarps) {
-    const int k = q < n0 ? W.q[par][0][q] : W.q[par][1][q - n0];
-    RadGeom rg;
-    rad_geom(C.g + 20L * k, C.G + 20L * k, rg);
-    const double *u0 = C.uu + (long)k * NVR, *p0 = C.pp + (long)k * NVR;
-    const double dt = C.dt[k];
-    ImpState s;
-    s.phase = PH_BASE;
-    s.j = 0;
-    s.sign = -1.;
-    s.xiapp = 1.;
-    s.evals = 0;
-    s.inner[0] = s.inner[1] = 0;
-    s.sw = W.wsw[k];
-    s.att = W.watt[k];
-    s.iter = W.wit[k];
-    s.warm = W.wwarm[k];
-    for (int i = 0; i < NVR; i++) s.pp[i] = W.wpp[(long)k * NVR + i];
-    const int warm0 = s.warm;
-    const double *wg = W.wguess + (long)k * NVR;
-    // what the state machine still evaluates itself (damped trials, the
-    // final inversion) runs its nested MHD inversion with the 32 lanes
-    // together: the tail's cells are the ones with the longest chains, so
-    // its latency is what counts (hard cells of a settled torus solve alone:
-    // 75.3 -> 65.4 ms)
-    ImpInner how{nullptr, 0u, true, warm_attempts};
-    int budget = 1 << 30;
-    int r;
-    while (true) {
-      if (s.phase == PH_BASE) {
-        if (lane < IMP_NCACHE) imp_eval_entry(R, u0, p0, dt, rg, s, lane, ce[lane]);
-        __syncwarp();
+      if (PRIM == IMP_MHD && !careful) {
+        // On MHD primitives a trial is kept or not by its energy alone (the
+        // verdict of the closure never rejects one), and a rejected trial
+        // leaves nothing but its radiation primitives, which the next
+        // inversion replaces: the rejected ones are counted and not
+        // evaluated.  Should the inversion of the trial that is kept end
+        // without replacing them, the trials are done again one by one
+        // (careful).
+        const double p0 = q.ppp[sh];
+        while (true) {
+          double x0 = p0;
+#pragma unroll
+          for (int j = 0; j < 4; j++) x0 -= xiapp * q.J[0][j] * q.f1[j];
+          if (x0 > p0 / R.maxdown && x0 < p0 * R.maxup) break;
+          if (x0 <= 0.) {
+            xiapp *= p0 / (p0 + fabs(x0));
+            xiapp *= 1.e-1;
+          } else {
+            xiapp /= R.dampfac;
+          }
+          rejected++;
+          if (!(xiapp >= R.maxdamping)) break;
+        }
       }
-      const ImpCache cache{ce, (1u << IMP_NCACHE) - 1u};
-      r = imp_advance(R, u0, p0, dt, rg, s, budget, wg, &how, &cache);
-      __syncwarp();   // every lane has read the entries before they are replaced
-      if (r != IMP_RUNNING) break;
+      // row `col` of the damped step
+      double xi = q.ppp[col + sh];
+#pragma unroll
+      for (int j = 0; j < 4; j++) xi -= xiapp * q.J[col][j] * q.f1[j];
+      x[0] = xi;
     }
-    if (lane == 0) {
-      if (r == IMP_DONE_OK) cell_success(R, C, k, rg, s.pp, s.att, s.iter);
-      else cell_failure(C, k);
-      atomicAdd(W.stats, (unsigned long long)((1 << 30) - budget));
-      if (warm0 && !s.warm) atomicAdd(W.stats + 2, 1ull);
-      atomicAdd(W.stats + 3, (unsigned long long)s.evals);
-      atomicAdd(W.stats + 4, (unsigned long long)s.inner[0]);
-      atomicAdd(W.stats + 5, (unsigned long long)s.inner[1]);
+#pragma unroll
+    for (int i = 3; i >= 0; i--) {
+      const double xi = __shfl_sync(FULL, x[0], i, 4);
+      if (i) x[i] = xi;
+      else x[0] = xi;
     }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned prev = atomicAdd(W.tail_done, 1u);
-    if (prev == gridDim.x - 1) {   // every block has read the counts: the queue is done
-      W.count[nq * 3 + 0] = 0;
-      W.count[nq * 3 + 1] = 0;
-      *W.tail_done = 0u;
-      atomicAdd(W.stats + 1, 1ull);
+    if (phase == PH_DAMP) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) pin[i + sh] = x[i];
     }
-  }
-}
-
-// The cooperative part of pass p: each cell whose evaluation was handed
-// over is taken by a whole warp, which repeats that evaluation and goes on
-// with the cell for the rest of the pass's budget, every nested MHD
-// inversion run by the 32 lanes together; the arithmetic is the same, so
-// the cell's results are too.  Unfinished cells join the next pass.
-__global__ void __launch_bounds__(128, KGPU_RAD_MIN_BLOCKS) k_rad_slow(RadParams R, Cell C, Work W, int n, int p, int K,
-                                                  int warm_attempts) {
-  const int ns0 = W.count[p * 3 + 2];
-  const int ns = ns0 < W.nslots ? ns0 : W.nslots;
-  const int par = p & 1;
-  const int lane = threadIdx.x & 31;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < ns; q += nwarps) {
-    const int k = W.qs[q];
-    ImpState s = W.ss[q];
-    RadGeom rg;
-    rad_geom(C.g + 20L * k, C.G + 20L * k, rg);
-    const double *u0 = C.uu + (long)k * NVR, *p0 = C.pp + (long)k * NVR;
-    const double dt = C.dt[k];
-    const double *wg = W.wguess + (long)k * NVR;
-    const int warm0 = s.warm;
-    const unsigned it0 = s.iter;
-    s.evals = 0;
-    s.inner[0] = s.inner[1] = 0;
-    int budget = K;
-    ImpInner how{nullptr, 0u, true, warm_attempts};
-    int r;
-    while ((r = imp_advance(R, u0, p0, dt, rg, s, budget, wg, &how)) == IMP_RUNNING) {
+    const bool spent = rejected > 0 && !(xiapp >= R.maxdamping);   // no trial is left
+    if (spent) act = false;
+    __syncwarp();   // every lane has read the iterate
+    if (phase == PH_BASE) {
+#pragma unroll
+      for (int i = 0; i < NVR; i++)
+        if ((i & 3) == col) q.ppp[i] = pin[i];
     }
-    if (lane == 0) {
-      atomicAdd(W.stats, (unsigned long long)(K - budget));
-      if (warm0 && !s.warm) atomicAdd(W.stats + 2, 1ull);
-      atomicAdd(W.stats + 3, (unsigned long long)s.evals);
-      atomicAdd(W.stats + 4, (unsigned long long)s.inner[0]);
-      atomicAdd(W.stats + 5, (unsigned long long)s.inner[1]);
-      if (r == IMP_PAUSE) {
-        const int type = imp_attempt(s.att, s.sw).prim;
-        const int at = atomicAdd(W.count + (p + 1) * 3 + type, 1);
-        W.q[par ^ 1][type][at] = k;
-        W.watt[k] = s.att;
-        W.wit[k] = s.iter;
-        W.wwarm[k] = s.warm;
-        for (int i = 0; i < NVR; i++) W.wpp[(long)k * NVR + i] = s.pp[i];
-      } else if (r == IMP_DONE_OK) {
-        cell_success(R, C, k, rg, s.pp, s.att, s.iter);
+    // the conserved state and the inversion of the other component
+    int corr = 0, u2pret = 0;
+    unsigned in0 = 0, in1 = 0;
+    if (PRIM == IMP_MHD) {
+      if (act) {
+        imp_rho_from_velocity(q.uu0, pin, rg.g);
+        imp_conserved(R, PRIM, q.uu0, pin, uu, rg);
+      }
+      together();
+      if (act) u2pret = u2p_rad(R, uu, pin, rg, corr);
+    } else {
+      U2PState us;
+      double Wc = 0.;
+      int r = 0, nit = 0;
+      // a warp with one live cell hands it to the 32 lanes at once
+      const unsigned live = __ballot_sync(FULL, act);
+      const bool lone = (live & ~(0xfu << ((__ffs(live | 0x80000000u) - 1) & ~3))) == 0u;
+      if (act) {
+        imp_conserved(R, PRIM, q.uu0, pin, uu, rg);
+        u2p_setup(uu, rg.g, us);
+        Wc = u2p_initial_w(R.gamma, pin, rg.g);
+      }
+      together();
+      if (act) {
+        r = u2p_solve_w(R.gamma, R.u2pconv, 0, us.c, Wc, nit, 1 << 30, 1 << 30, &in1,
+                        cap && lone && phase != PH_JAC ? 1u : cap);
+      }
+      // inversions over the cap, one after another: the 32 lanes go on with
+      // each, trying the damped points of a step together.  The four lanes
+      // of a quad share one, except in a Jacobian trip
+      unsigned over = __ballot_sync(FULL, r == U2P_OVER_CAP);
+      while (over) {
+        const int L = __ffs(over) - 1;
+        U2PCons c;
+        c.Qn = __shfl_sync(FULL, us.c.Qn, L);
+        c.Qt2 = __shfl_sync(FULL, us.c.Qt2, L);
+        c.D = __shfl_sync(FULL, us.c.D, L);
+        c.QdotBsq = __shfl_sync(FULL, us.c.QdotBsq, L);
+        c.Bsq = __shfl_sync(FULL, us.c.Bsq, L);
+        c.Sc = 0.;   // the entropy equation's, not read
+        double Wb = __shfl_sync(FULL, Wc, L);
+        int itb = __shfl_sync(FULL, nit, L);
+        const int rb = u2p_newton_warp(R.gamma, R.u2pconv, 0, c, Wb, itb);
+        if (r == U2P_OVER_CAP && (lane == L || (quad == (L >> 2) && phase != PH_JAC))) {
+          r = rb;
+          Wc = Wb;
+          nit = itb;
+        }
+        if (lane == L) st[6]++;
+        over = __ballot_sync(FULL, r == U2P_OVER_CAP);
+      }
+      together();
+      if (act) {
+        in0 = (unsigned)nit;
+        if (r == 0) r = u2p_final(R.gamma, us, Wc, nit, uu, pin, rg.g, false);
+        u2pret = r < 0 ? -2 : 0;
+      }
+    }
+    // a trial: kept or damped further (see imp_advance)
+    bool fail = false, resid = act, chained = false;
+    if (have && phase == PH_DAMP && (spent || (PRIM == IMP_MHD && rejected > 0 && u2pret < 0))) {
+      resid = false;
+      if (spent) {
+        fail = true;
+        if (col == 0) st[3] += rejected;
       } else {
-        cell_failure(C, k);
+        xiapp = 1.;
+        careful = true;
+      }
+    } else if (have && phase == PH_DAMP) {
+      if (col == 0) {
+        st[3] += 1 + rejected;
+        st[4] += in0;
+        st[5] += in1;
+      }
+      resid = false;
+#pragma unroll
+      for (int i = 0; i < NVR; i++)
+        if ((i & 3) == col) q.pp[i] = pin[i];
+      const double p0 = q.ppp[sh];
+      if (x[0] > p0 / R.maxdown && x[0] < p0 * R.maxup && ((PRIM == IMP_MHD && corr > 0) || u2pret >= -1)) {
+        if (iter > R.maxiter) {
+          fail = true;
+        } else {
+          phase = PH_BASE;
+          if (PRIM == IMP_MHD && P.eq == IMP_ENERGY) {
+            iter++;
+            resid = chained = true;
+          }
+        }
+      } else {
+        if (x[0] <= 0.) {
+          xiapp *= p0 / (p0 + fabs(x[0]));
+          xiapp *= 1.e-1;
+        } else {
+          xiapp /= R.dampfac;
+        }
+        if (!(xiapp >= R.maxdamping)) fail = true;
       }
     }
-    (void)it0;
+    together();   // ppp[sh] has been read in every lane of the quad
+    double f[4] = {0., 0., 0., 0.}, err = 0.;
+    int fret = 0;
+    if (resid) {
+      if (chained) {   // the next iteration starts from the kept trial
+#pragma unroll
+        for (int i = 0; i < NVR; i++)
+          if ((i & 3) == col) q.ppp[i] = pin[i];
+      }
+      fret = imp_residual(R, P, pin, uu, q.uu0, q.pp00, q.Ehat0, q.dt, rg, u2pret, corr, f, err);
+    }
+    together();
+    bool done = false;
+    if (resid && phase == PH_BASE) {
+      if (col == 0) {
+        st[0]++;
+        st[3]++;
+        st[4] += in0;
+        st[5] += in1;
+      }
+      if (fret < 0) {
+        fail = true;
+      } else if (err < (P.eq == IMP_ENTROPY ? R.entrconv : R.conv)) {
+        if (iter > R.maxiter) {
+          fail = true;
+        } else {
+          // the final inversion is this evaluation's (see imp_advance)
+          if (col == 0) {
+            st[3]++;
+            st[4] += in0;
+            st[5] += in1;
+          }
+          if ((PRIM == IMP_MHD && corr > 0) || u2pret < -1) fail = true;
+          else done = true;
+        }
+      } else {
+        if (col == 0) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) q.f1[i] = f[i];
+        }
+        phase = PH_JAC;
+        todo = minus = true;
+        cin0 = cin1 = 0;
+        resid = false;
+      }
+    }
+    __syncwarp();
+    // Jacobian: a column that fails on one side is tried on the other; the
+    // attempt fails at the first column that fails on both
+    const bool jac = resid && phase == PH_JAC;   // this lane evaluated its column in this trip
+    bool dead = false;
+    if (jac) {
+      cin0 += in0;
+      cin1 += in1;
+      if (fret < 0) {
+        dead = !minus;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) q.J[i][col] = (f[i] - q.f1[i]) / (pick4(pin + sh, col) - q.ppp[col + sh]);
+        todo = false;
+      }
+    }
+    const unsigned mjac = __ballot_sync(FULL, jac) >> (quad * 4) & 0xfu;
+    if (__any_sync(FULL, jac)) {
+      const unsigned mdead = __ballot_sync(FULL, dead) >> (quad * 4) & 0xfu;
+      const unsigned mopen = __ballot_sync(FULL, jac && todo && !dead) >> (quad * 4) & 0xfu;
+      __syncwarp();
+      if (mjac) {
+        if (mdead || !mopen) {
+          // evaluations as the one-lane sequence counts them: the columns up
+          // to the first that fails, two where the first side failed
+          const int last = mdead ? __ffs(mdead) - 1 : 3;
+          if (col <= last) {
+            st[3] += minus ? 1u : 2u;
+            st[4] += cin0;
+            st[5] += cin1;
+          }
+          if (mdead) {
+            fail = true;
+          } else {
+            double a[4][4], ia[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+              for (int j = 0; j < 4; j++) a[i][j] = q.J[i][j];
+            if (inverse_44(a, ia) < 0) {
+              fail = true;
+            } else {
+              __syncwarp(0xfu << (quad * 4));
+#pragma unroll
+              for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                  if (j == col) q.J[i][j] = ia[i][j];
+              xiapp = 1.;
+              careful = false;
+              phase = PH_DAMP;
+            }
+          }
+        } else if (todo) {
+          minus = false;
+        }
+      }
+    }
+    // the end of an attempt
+    if (done) {
+#pragma unroll
+      for (int i = 0; i < NVR; i++)
+        if ((i & 3) == col) C.pp_out[(long)k * NVR + i] = pin[i];
+      if (col == 0) {
+        C.status[k] = 0;
+        C.attempt[k] = att;
+        C.iters[k] = iter;
+      }
+      have = false;
+    } else if (have && fail) {
+      att++;
+      if (warm && att >= warm_attempts) {
+        warm = 0;
+        att = 0;
+        if (col == 0) st[2]++;
+      }
+      if (att >= IMP_NATTEMPTS) {
+        if (col == 0) C.status[k] = -1;
+        have = false;
+      } else {
+        const ImpParams N = imp_attempt(att, sw);
+        if (N.prim != PRIM || N.frame != FRAME) {
+          if (col == 0) quad_push(Q.l[N.frame * 2 + N.prim], quad_entry(k, att, warm, sw));
+          have = false;
+        } else {
+          begin = true;
+        }
+      }
+    }
     __syncwarp();
   }
 }
 
+// The resident kernel of the batched form.  A block chooses a kind of attempt
+// that has cells waiting and works on it until its list is empty and its own
+// cells are done, then chooses again; it leaves when every list is empty (a
+// cell on its way to another list is then some other block's, which will look
+// there itself).  No attempt waits for the slowest cell of the one before.
+//
+// What bounds it is the fetch of its instructions: each kind of attempt is a
+// loop of about 110 to 150 KB of code, and warps that are at different places
+// of it evict one another's from the instruction cache (21 cycles of "no
+// instruction" per issue with 16 warps an SM running free, of 40).  So the
+// blocks of an SM work on the same kind of attempt while it has cells (the
+// SMs are shared out between the primitives by the cells that start on
+// either), and the warps of a block go through a trip in step, meeting at five
+// barriers.  262144 cells of the batched-solve distribution, of which a fifth
+// runs through several attempts, from the cell's own guess / the network's:
+// warps running free 162 / 216 ms, in step in blocks of 4 warps 117 / 162 ms,
+// of 8 104 / 123 ms, of 16 112 / 106 ms.  With one cell a warp there is
+// little to share and much to wait for (1537 cells: 16 ms free, 18 in step),
+// so such a block runs free.
+//
+// Before (passes over queues of cells, one lane a cell, a launch per pass and
+// for the cells that need whole warps): 363 / 288 ms, and 23 ms for 1537.
+__global__ void __launch_bounds__(32 * QUAD_WARPS, QUAD_BLOCKS)
+    k_rad_quads(RadParams R, Cell C, Work W, QuadLists Q, int *sm_role, int sms, unsigned cap, int warm_attempts) {
+  extern __shared__ __align__(16) unsigned char quad_smem[];
+  QuadCell (*cells)[QUAD_CELLS] = reinterpret_cast<QuadCell(*)[QUAD_CELLS]>(quad_smem);
+  __shared__ int choice[2];
+  const int wib = threadIdx.x >> 5;
+  unsigned smid;
+  asm("mov.u32 %0, %%smid;" : "=r"(smid));
+  unsigned st[7] = {0, 0, 0, 0, 0, 0, 0};
+  while (true) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int a[4], start[2] = {0, 0};
+      for (int i = 0; i < 4; i++) {
+        a[i] = *(volatile int *)Q.l[i].avail;
+        start[i & 1] += W.count[i];
+      }
+      int split = (int)((long)sms * start[0] / (start[0] + start[1]));   // SMs for radiation primitives
+      if (start[0] > 0 && split == 0) split = 1;
+      if (start[1] > 0 && split == sms) split = sms - 1;
+      // what the other blocks of this SM are at, while it has cells; else the
+      // longer list of this SM's primitives, else of the others
+      volatile int *smr = sm_role + smid;
+      int r = *smr - 1;
+      if (r < 0 || a[r] <= 0) {
+        const int p = (int)smid < split ? 0 : 1;
+        r = a[p] >= a[2 + p] ? p : 2 + p;
+        if (a[r] <= 0) r = a[p ^ 1] >= a[2 + (p ^ 1)] ? (p ^ 1) : 2 + (p ^ 1);
+        if (a[r] <= 0) r = -1;
+        else *smr = r + 1;
+      }
+      const int warps = (int)gridDim.x * QUAD_WARPS;
+      choice[0] = r;
+      // few cells are spread over the warps
+      choice[1] = r < 0 ? 0 : (a[r] >= QUAD_CELLS * warps ? QUAD_CELLS : (a[r] + warps - 1) / warps);
+    }
+    __syncthreads();
+    const int r = choice[0], per = choice[1];
+    if (r < 0) break;
+    if (r == 0) quads_run<IMP_RAD, IMP_LAB>(R, C, W, Q, cells[wib], per, per > 1, cap, warm_attempts, st);
+    else if (r == 1) quads_run<IMP_MHD, IMP_LAB>(R, C, W, Q, cells[wib], per, per > 1, cap, warm_attempts, st);
+    else if (r == 2) quads_run<IMP_RAD, IMP_FF>(R, C, W, Q, cells[wib], per, per > 1, cap, warm_attempts, st);
+    else quads_run<IMP_MHD, IMP_FF>(R, C, W, Q, cells[wib], per, per > 1, cap, warm_attempts, st);
+  }
+  for (int i = 0; i < 7; i++)
+    if (i != 1) warp_add(W.stats + i, st[i]);
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(W.stats + 1, 1ull);
+}
+
+// The outputs of every cell: the entropy and the conserved variables of a
+// solution (p2u at the end of solve_implicit_lab, rad.c:1525-1540), or the
+// state kept where every attempt failed.  On its own so that the solver's
+// kernel does not carry this code.
+__global__ void __launch_bounds__(128) k_rad_outputs(RadParams R, Cell C, int n) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  if (C.status[k] != 0) {
+    cell_failure(C, k);
+    return;
+  }
+  RadGeom rg;
+  rad_geom(C.g + 20L * k, C.G + 20L * k, rg);
+  double pw[NVR];
+  for (int i = 0; i < NVR; i++) pw[i] = C.pp_out[(long)k * NVR + i];
+  pw[ENTR] = rad_Sfromu(R, pw[RHO], pw[UU]);
+  cell_success(R, C, k, rg, pw, C.attempt[k], C.iters[k]);
+}
+
+constexpr int TAIL_WARPS = 4;   // warps per block of 128
 // The persistent form.  A lane's cell state at the start of a Newton
 // iteration: what the per-cell work arrays hold (k_rad_start, or a cell
 // paused at an iteration boundary).
@@ -888,7 +1234,7 @@ extern "C" int kgpu_rad_set_pass_iters(int k) {
 
 extern "C" size_t kgpu_rad_work_bytes(int n) {
   if (n < 0) return 0;
-  return work_layout(n, kMaxPasses, nullptr, nullptr) + 256;
+  return work_layout(n, nullptr, nullptr) + 256;
 }
 
 // resident blocks of k_rad_persist per SM
@@ -900,12 +1246,10 @@ static int persist_blocks_per_sm(const Opts &o) {
 }
 
 // kernels one solve launches (for the launch counters)
-static long long solve_launches(const RadParams &R, int mode, const Opts &o, bool have_prev) {
+static long long solve_launches(int mode) {
   if (mode == KGPU_RAD_PLAIN) return 1;
   if (mode == KGPU_RAD_PERSISTENT) return 3;
-  const int np = max_passes(R, o.pass_iters);
-  const bool count = have_prev && np > 1 && o.tail > 0 && o.hard >= 0;   // k_rad_count_hard
-  return 1 + (count ? 1 : 0) + (o.inner_cap ? 2 : 1) * np + (o.tail ? np - 1 : 0);
+  return 4;
 }
 
 // acc (device, optional): counters the solve adds to instead of reporting
@@ -918,7 +1262,7 @@ static int rad_solve_device(int n, const kgpu_rad_params *rp, const double *uu, 
                             const double *G, const double *dt, const float *ypred, double *pp_out, double *uu_out,
                             int *status, int *attempt, int *iters, int mode, void *work, void *stream,
                             unsigned long long *stats, int nstats, const Opts &o, unsigned long long *acc = nullptr,
-                            int gate = -1, bool have_prev = false) {
+                            int gate = -1) {
   if (n < 0 || !rp || (mode != KGPU_RAD_PLAIN && mode != KGPU_RAD_BATCHED && mode != KGPU_RAD_PERSISTENT))
     return KGPU_EINVAL;
   if (n > 0 && (!uu || !pp || !g || !G || !dt || !pp_out || !uu_out || !status || !attempt || !iters))
@@ -951,23 +1295,26 @@ static int rad_solve_device(int n, const kgpu_rad_params *rp, const double *uu, 
     }
     return 0;
   }
-  const int K = o.pass_iters;
-  const int passes = mode == KGPU_RAD_BATCHED ? max_passes(R, K) : 1;
   char *base = (char *)(((uintptr_t)work + 255) & ~(uintptr_t)255);
   Work W;
-  work_layout(n, passes, &W, base);   // fits: the area is sized for kMaxPasses >= passes
-  RCK(cudaMemsetAsync(W.count, 0, (size_t)(passes + 2) * 3 * 4, st));
+  work_layout(n, &W, base);
+  RCK(cudaMemsetAsync(W.count, 0, (size_t)kCounters * 4, st));
   RCK(cudaMemsetAsync(W.tail_done, 0, sizeof(unsigned), st));
   RCK(cudaMemsetAsync(W.ctl, 0, 4 * sizeof(unsigned), st));
   if (acc) W.stats = acc;
   else RCK(cudaMemsetAsync(W.stats, 0, 8 * sizeof(unsigned long long), st));
-  const int hard = (have_prev && mode == KGPU_RAD_BATCHED && passes > 1 && o.tail > 0) ? o.hard : -1;
-  const int limit = sm_count() * o.tail * 4;
-  if (hard >= 0) {
-    k_rad_count_hard<<<(n + 127) / 128, 128, 0, st>>>(C, n, hard, W.ctl);
-    RCK(cudaGetLastError());
+  // the batched form's lists lie in wpp, which only the persistent one uses
+  QuadLists Q;
+  {
+    unsigned long long *e = (unsigned long long *)W.wpp;
+    static_assert(2 * (QUAD_LAB_TURNS + QUAD_FF_TURNS) <= NVR, "the lists fit");
+    for (int i = 0; i < 4; i++) {
+      Q.l[i] = QuadList{e, W.count + 8 + i, W.count + 16 + i, W.count + 24 + i};
+      e += (size_t)n * (i < 2 ? QUAD_LAB_TURNS : QUAD_FF_TURNS);
+    }
+    if (mode == KGPU_RAD_BATCHED) RCK(cudaMemsetAsync(W.wpp, 0, (size_t)((char *)e - (char *)W.wpp), st));
   }
-  k_rad_start<<<(n + 127) / 128, 128, 0, st>>>(R, C, W, n, ypred, gate, o.skip, hard, limit);
+  k_rad_start<<<(n + 127) / 128, 128, 0, st>>>(R, C, W, Q, n, ypred, gate, o.skip, mode == KGPU_RAD_PERSISTENT);
   RCK(cudaGetLastError());
   if (mode == KGPU_RAD_PERSISTENT) {
     const int grid = sm_count() * persist_blocks_per_sm(o);
@@ -976,23 +1323,20 @@ static int rad_solve_device(int n, const kgpu_rad_params *rp, const double *uu, 
     k_rad_finish<<<grid, 128, 0, st>>>(R, C, W, o.warm_attempts, (unsigned)o.inner_cap);
     RCK(cudaGetLastError());
   } else {
-    const int grid = sm_count() * 8;
-    for (int p = 0; p < passes; p++) {
-      const int Kp = p == passes - 1 ? (1 << 30) : K;   // the last pass finishes whatever is left
-      const int blocks = p == 0 ? (n + 127) / 128 : grid;
-      k_rad_pass<<<blocks, 128, 0, st>>>(R, C, W, n, p, Kp, (unsigned)o.inner_cap, o.warm_attempts);
-      RCK(cudaGetLastError());
-      if (o.inner_cap) {
-        k_rad_slow<<<grid / 2, 128, 0, st>>>(R, C, W, n, p, Kp, o.warm_attempts);
-        RCK(cudaGetLastError());
-      }
-      if (o.tail && p < passes - 1) {
-        // o.tail blocks of four warps per SM, one cell per warp at a time;
-        // it takes over once the unfinished cells are no more than its warps
-        k_rad_tail<<<sm_count() * o.tail, 128, 0, st>>>(R, C, W, n, p, sm_count() * o.tail * 4, o.warm_attempts);
-        RCK(cudaGetLastError());
-      }
-    }
+    k_rad_lists<<<1, 32, 0, st>>>(Q, W.count);
+    RCK(cudaGetLastError());
+    const int sms = sm_count();
+    // handing an inversion over costs no more than its last evaluation here, so
+    // it is done early: 16 evaluations by default (a fifth of the lanes of a
+    // warp would wait for the others at 64: 115 against 104 ms for 262144 cells)
+    const unsigned cap = o.inner_cap > 0 ? (unsigned)(o.inner_cap + 3) / 4u : 0u;
+    constexpr int kQuadSmem = QUAD_WARPS * QUAD_CELLS * (int)sizeof(QuadCell);
+    RCK(cudaFuncSetAttribute(k_rad_quads, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuadSmem));
+    k_rad_quads<<<sms * QUAD_BLOCKS, 32 * QUAD_WARPS, kQuadSmem, st>>>(R, C, W, Q, W.count + 64, sms, cap,
+                                                                      o.warm_attempts);
+    RCK(cudaGetLastError());
+    k_rad_outputs<<<(n + 127) / 128, 128, 0, st>>>(R, C, n);
+    RCK(cudaGetLastError());
   }
   if (stats) {
     RCK(cudaMemcpyAsync(stats, W.stats, nstats * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
@@ -1008,9 +1352,9 @@ int kgpu_rad_solve_enqueue(int n, const kgpu_rad_params *rp, const double *uu, c
                            int *status, int *attempt, int *iters, int mode, void *work, void *stream,
                            unsigned long long *acc, long long *launches, int gate, const kgpu_rad_solver_opts *opts) {
   const Opts o = opts ? from_api(*opts) : g_opts;
-  if (launches) *launches = solve_launches(to_dev(*rp), mode, o, true);
+  if (launches) *launches = solve_launches(mode);
   return rad_solve_device(n, rp, uu, pp, g, G, dt, ypred, pp_out, uu_out, status, attempt, iters, mode, work, stream,
-                          nullptr, 0, o, acc, gate, true);
+                          nullptr, 0, o, acc, gate);
 }
 
 bool kgpu_rad_opts_valid(const kgpu_rad_solver_opts &o) { return opts_valid(o); }

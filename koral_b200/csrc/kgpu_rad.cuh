@@ -23,6 +23,9 @@
 #define KG_RAD_CALL
 #endif
 
+// rare branches of the evaluations, kept out of their instruction stream
+#define KG_COLD static __host__ __device__ __noinline__
+
 namespace kgpu {
 
 constexpr int NVR = 13;
@@ -78,7 +81,7 @@ KG_HD double rad_kappa_abs(const RadParams &R, const double *pp) {
   double rho = pp[RHO];
   double T = peq_T_from_urho(R, pp[UU], pp[RHO]);
   double rhocgs = rho / R.ggg * R.ccc * R.ccc / R.masscm / R.masscm;
-  return R.kramers * rhocgs * pow(T, -3.5) / R.ggg * R.ccc * R.ccc / R.masscm * rho;
+  return R.kramers * rhocgs * pow_call(T, -3.5) / R.ggg * R.ccc * R.ccc / R.masscm * rho;
 }
 KG_HD double rad_kappa_es(const RadParams &R, const double *pp) { return R.kes_gu * pp[RHO]; }
 
@@ -284,6 +287,35 @@ KG_RAD_CALL KG_HD void m1_cold(const RadGeom &rg, double Avcon[4], double Avcov[
   }
 }
 
+// The two cold solutions, at rest and at the largest Lorentz factor, of
+// which the closer one is taken where the closure has no solution
+// (u2prad.c:251-411).  Out of line on the device: rare, and as long as the
+// closure itself, it would spread every evaluation of the implicit solve
+// over more of the instruction cache.
+struct M1Cold {
+  double Erf, gammarel2, urf[3];
+};
+KG_COLD M1Cold m1_corrected(const RadParams &R, const RadGeom &rg, double A0, double A1, double A2, double A3) {
+  const double gammamax = R.gammamaxrad;
+  const double gam2[2] = {pow(1.0 + 10.0 * R.numepsilon, 2.0), gammamax * gammamax};   // slow, fast
+  M1Cold s{}, f{};
+  double ds = 0.;
+#pragma unroll 1
+  for (int i = 0; i < 2; i++) {
+    double con[4] = {0., 0., 0., 0.}, cov[4] = {A0, A1, A2, A3}, u[4] = {0., 0., 0., 0.}, E;
+    m1_cold(rg, con, cov, i == 0 ? gam2[0] : gam2[1], E, u);
+    const double d = fabs(cov[0] - A0);
+    const M1Cold c{E, i == 0 ? gam2[0] : gam2[1], {u[1], u[2], u[3]}};
+    if (i == 0) {
+      s = c;
+      ds = d;
+    } else {
+      f = ds > d ? c : s;
+    }
+  }
+  return f;
+}
+
 // u2p_rad (u2prad.c:485-520 with get_m1closure_* 116-411).  Returns 0 or -1;
 // corrected = 1 when the closure fell back to a cold solution.
 KG_RAD_CALL KG_HD int u2p_rad(const RadParams &R, const double *uu, double *pp, const RadGeom &rg, int &corrected) {
@@ -305,25 +337,10 @@ KG_RAD_CALL KG_HD int u2p_rad(const RadParams &R, const double *uu, double *pp, 
     for (int ii = 0; ii < 4; ii++)
       urf[ii] = alpha * (Avcon[ii] + 1. / 3. * Erf * GG[0][ii] * (4.0 * gammarel2 - 1.0)) / (4. / 3. * Erf * gammarel);
   } else {
-    double gs2 = pow(1.0 + 10.0 * R.numepsilon, 2.0);
-    double cs[4], ks[4], us[4] = {0., 0., 0., 0.}, Es;
-    double cf[4], kf[4], uf[4] = {0., 0., 0., 0.}, Ef;
-    for (int j = 0; j < 4; j++) {
-      cs[j] = cf[j] = Avcon[j];
-      ks[j] = kf[j] = Avcov[j];
-    }
-    m1_cold(rg, cs, ks, gs2, Es, us);
-    double gf2 = gammamax * gammamax;
-    m1_cold(rg, cf, kf, gf2, Ef, uf);
-    if (fabs(ks[0] - Avcov[0]) > fabs(kf[0] - Avcov[0])) {
-      for (int j = 0; j < 4; j++) urf[j] = uf[j];
-      gammarel2 = gf2;
-      Erf = Ef;
-    } else {
-      for (int j = 0; j < 4; j++) urf[j] = us[j];
-      gammarel2 = gs2;
-      Erf = Es;
-    }
+    const M1Cold c = m1_corrected(R, rg, Avcov[0], Avcov[1], Avcov[2], Avcov[3]);
+    for (int j = 1; j < 4; j++) urf[j] = c.urf[j - 1];
+    gammarel2 = c.gammarel2;
+    Erf = c.Erf;
     corrected = 1;
   }
   if (!isfinite(Erf) || !isfinite(gammarel2) || !isfinite(urf[1]) || !isfinite(urf[2]) || !isfinite(urf[3]))
@@ -417,32 +434,41 @@ KG_RAD_CALL KG_HD int imp_u2p_hot(const RadParams &R, const double *uu, double *
 KG_HD double rad_Sfromu(const RadParams &R, double rho, double u) { return calc_Sfromu(R.gamma, rho, u); }
 
 // Conserved state that goes with the primitives pp when the other
-// component takes the opposite change of energy-momentum, and the inversion
-// of that other component (rad.c:140-198 and 883-960).  Returns u2p's
-// verdict as the residual sees it: 0 or -1 usable, -2 failed; corr set
-// when the M1 closure was corrected.
-KG_HD int imp_counterpart(const RadParams &R, int prim, const double *uu0, double *pp, double *uu, const RadGeom &rg,
-                          int &corr, const ImpInner *inner = nullptr) {
+// component takes the opposite change of energy-momentum (rad.c:140-198 and
+// 883-960)
+KG_HD void imp_conserved(const RadParams &R, int prim, const double *uu0, const double *pp, double *uu,
+                         const RadGeom &rg) {
   Grid G;
   G.gamma = R.gamma;
   G.nv = NVMAX;
   p2u_rad_full(G, pp, uu, rg.g);
   uu[ENTR] = uu0[ENTR] - (uu[EE0] - uu0[EE0]);
-  corr = 0;
   if (prim == IMP_RAD) {
     uu[RHO] = uu0[RHO];
     uu[1] = uu0[1] - (uu[EE0] - uu0[EE0]);
     uu[2] = uu0[2] - (uu[FX0] - uu0[FX0]);
     uu[3] = uu0[3] - (uu[FY0] - uu0[FY0]);
     uu[4] = uu0[4] - (uu[FZ0] - uu0[FZ0]);
+  } else {
+    uu[EE0] = uu0[EE0] - (uu[1] - uu0[1]);
+    uu[FX0] = uu0[FX0] - (uu[2] - uu0[2]);
+    uu[FY0] = uu0[FY0] - (uu[3] - uu0[3]);
+    uu[FZ0] = uu0[FZ0] - (uu[4] - uu0[4]);
+  }
+}
+
+// imp_conserved and the inversion of the other component.  Returns u2p's
+// verdict as the residual sees it: 0 or -1 usable, -2 failed; corr set
+// when the M1 closure was corrected.
+KG_HD int imp_counterpart(const RadParams &R, int prim, const double *uu0, double *pp, double *uu, const RadGeom &rg,
+                          int &corr, const ImpInner *inner = nullptr) {
+  imp_conserved(R, prim, uu0, pp, uu, rg);
+  corr = 0;
+  if (prim == IMP_RAD) {
     const int r = imp_u2p_hot(R, uu, pp, rg.g, inner);
     if (r == U2P_OVER_CAP) return r;
     return r < 0 ? -2 : 0;
   }
-  uu[EE0] = uu0[EE0] - (uu[1] - uu0[1]);
-  uu[FX0] = uu0[FX0] - (uu[2] - uu0[2]);
-  uu[FY0] = uu0[FY0] - (uu[3] - uu0[3]);
-  uu[FZ0] = uu0[FZ0] - (uu[4] - uu0[4]);
   return u2p_rad(R, uu, pp, rg, corr);
 }
 
@@ -468,12 +494,24 @@ KG_HD int imp_prepare(const RadParams &R, const ImpParams &P, const double *uu0,
   return imp_counterpart(R, P.prim, uu0, pp, uu, rg, corr, inner);
 }
 
+// fluid-frame radiation energy density of the primitives pp
+KG_HD double imp_Ehat(const double *pp, const Geom &g) {
+  double ucon[4], Rtt;
+  calc_ff_Rtt(pp, g, Rtt, ucon);
+  return -Rtt;
+}
+
+KG_HD double imp_Ehat0(const ImpParams &P, const double *pp00, const Geom &g) {
+  return P.frame == IMP_FF && P.prim == IMP_RAD ? imp_Ehat(pp00, g) : 0.;
+}
+
 // residual f[4] and its relative size from a prepared state (the rest of
-// f_implicit_lab_4dprim, rad.c:199-351).  Returns -1 on failure, 1 when the
-// closure was corrected, else 0.
+// f_implicit_lab_4dprim, rad.c:199-351).  Ehat0: imp_Ehat of the cell's
+// guess pp00 (read in the fluid frame on radiation primitives only).
+// Returns -1 on failure, 1 when the closure was corrected, else 0.
 KG_RAD_CALL KG_HD int imp_residual(const RadParams &R, const ImpParams &P, double *pp, const double *uu, const double *uu0,
-                       const double *pp00, double dt, const RadGeom &rg, int u2pret, int corr, double f[4],
-                       double &err0) {
+                       const double *pp00, double Ehat0, double dt, const RadGeom &rg, int u2pret, int corr,
+                       double f[4], double &err0) {
   const Geom &g = rg.g;
   const double gdetu = g.gdet;
   int ret = corr != 0 ? 1 : 0;
@@ -516,14 +554,11 @@ KG_RAD_CALL KG_HD int imp_residual(const RadParams &R, const ImpParams &P, doubl
     else
       err[0] = 0.;
   } else {
-    double pp0[NVR];
-    for (int i = 0; i < NVR; i++) pp0[i] = pp00[i];
+    const double *pp0 = pp00;
     calc_Gi(R, pp, g, Gi, 0);
-    double uconf[4], Rtt0, Rtt;
-    calc_ff_Rtt(pp0, g, Rtt0, uconf);
+    double uconf[4], Rtt;
     calc_ff_Rtt(pp, g, Rtt, uconf);
     double Ehat = -Rtt;
-    double Ehat0 = -Rtt0;
     double dtau = dt / uconf[0];
     if (P.prim == IMP_RAD) {
       if (P.eq == IMP_ENERGY) {
@@ -539,10 +574,10 @@ KG_RAD_CALL KG_HD int imp_residual(const RadParams &R, const ImpParams &P, doubl
         f[0] = pp[UU] - pp0[UU] - dtau * Gi[0];
         err[0] = fabs(f[0]) / (fabs(pp[UU]) + fabs(pp0[UU]) + fabs(dtau * Gi[0]));
       } else {
-        pp0[ENTR] = rad_Sfromu(R, pp0[RHO], pp0[UU]);
+        const double S0 = rad_Sfromu(R, pp0[RHO], pp0[UU]);
         pp[ENTR] = rad_Sfromu(R, pp[RHO], pp[UU]);
-        f[0] = pp[ENTR] - pp0[ENTR] - dtau * Gi[0];
-        err[0] = fabs(f[0]) / (fabs(pp[ENTR]) + fabs(pp0[ENTR]) + fabs(dtau * Gi[0]));
+        f[0] = pp[ENTR] - S0 - dtau * Gi[0];
+        err[0] = fabs(f[0]) / (fabs(pp[ENTR]) + fabs(S0) + fabs(dtau * Gi[0]));
       }
     }
   }
@@ -590,9 +625,12 @@ KG_HD int imp_startwith(const RadParams &R, const double *pp0, const Geom &g) {
 // are common to all of them, the residual is added for base and Jacobian
 // evaluations — and then moves the cell's state to the next one, so all
 // lanes of a warp run the expensive part together whatever phase their cell
-// is in.  The sequence of operations per cell is the reference's.
+// is in.  The sequence of operations per cell is the reference's, but for
+// evaluations whose inputs are those of the one before (the final inversion,
+// and on MHD primitives the base after an accepted trial), which are not
+// repeated.
 // ---------------------------------------------------------------------------
-enum ImpPhase { PH_BASE = 0, PH_JAC = 1, PH_DAMP = 2, PH_FINAL = 3 };
+enum ImpPhase { PH_BASE = 0, PH_JAC = 1, PH_DAMP = 2 };
 enum ImpAdvance { IMP_RUNNING = 0, IMP_DONE_OK = 1, IMP_DONE_FAIL = 2, IMP_PAUSE = 3, IMP_OVER_CAP = 4 };
 
 struct ImpState {
@@ -667,6 +705,17 @@ struct ImpCache {
   unsigned valid;   // bit i: entry i present
 };
 
+// The finite-difference step of Jacobian column j, variable value x, on the
+// side `sign`
+KG_HD double imp_fd_step(const RadParams &R, int j, double sign, double x, const Geom &g) {
+  if (j == 0) return sign * R.eps * x;
+  double sg = x > 0. ? 1. : (x < 0. ? -1. : (x == 0. ? 1. : 0.));
+  double lim = 1.e-6 / sqrt(g.gg[j][j]);
+  double ax = fabs(x);
+  double veleps = R.eps * sg * (lim > ax ? lim : ax);
+  return x >= 0. ? sign * veleps : -sign * veleps;
+}
+
 // The input of an evaluation in phase PH_BASE or PH_JAC (column s.j on side
 // s.sign), as imp_advance forms it.
 KG_HD void imp_input(const RadParams &R, int sh, const ImpState &s, const RadGeom &rg, double *pin) {
@@ -676,17 +725,7 @@ KG_HD void imp_input(const RadParams &R, int sh, const ImpState &s, const RadGeo
   }
   for (int i = 0; i < NVR; i++) pin[i] = s.ppp[i];
   const int j = s.j;
-  double del;
-  if (j == 0) {
-    del = s.sign * R.eps * s.ppp[sh];
-  } else {
-    double x = s.ppp[j + sh];
-    double sg = x > 0. ? 1. : (x < 0. ? -1. : (x == 0. ? 1. : 0.));
-    double lim = 1.e-6 / sqrt(rg.g.gg[j][j]);
-    double ax = fabs(x);
-    double veleps = R.eps * sg * (lim > ax ? lim : ax);
-    del = x >= 0. ? s.sign * veleps : -s.sign * veleps;
-  }
+  const double del = imp_fd_step(R, j, s.sign, s.ppp[j + sh], rg.g);
   pin[j + sh] = s.ppp[j + sh] + del;
 }
 
@@ -716,7 +755,7 @@ KG_HD bool imp_eval_entry(const RadParams &R, const double *uu0, const double *p
   if (e.u2pret == U2P_OVER_CAP) return false;
   for (int i = 0; i < 4; i++) e.f[i] = 0.;
   e.err = 0.;
-  e.fret = imp_residual(R, P, e.pin, uu, uu0, pp00, dt, rg, e.u2pret, e.corr, e.f, e.err);
+  e.fret = imp_residual(R, P, e.pin, uu, uu0, pp00, imp_Ehat0(P, pp00, rg.g), dt, rg, e.u2pret, e.corr, e.f, e.err);
   return true;
 }
 
@@ -743,7 +782,7 @@ KG_HD int imp_advance(const RadParams &R, const double *uu0, const double *pp00,
     imp_input(R, sh, s, rg, pin);
   } else if (s.phase == PH_JAC) {
     imp_input(R, sh, s, rg, pin);
-  } else if (s.phase == PH_DAMP) {
+  } else {
     double xxx[4];
     for (int i = 0; i < 4; i++) xxx[i] = s.ppp[i + sh];
     for (int i = 0; i < 4; i++)
@@ -751,8 +790,6 @@ KG_HD int imp_advance(const RadParams &R, const double *uu0, const double *pp00,
     for (int i = 0; i < NVR; i++) pin[i] = s.pp[i];
     for (int i = 0; i < 4; i++) pin[i + sh] = xxx[i];
     xxx0 = xxx[0];
-  } else {
-    for (int i = 0; i < NVR; i++) pin[i] = s.pp[i];
   }
   // the evaluation: other component's inversion, residual where needed
   const int wa = how ? how->warm_attempts : IMP_NATTEMPTS;
@@ -761,6 +798,7 @@ KG_HD int imp_advance(const RadParams &R, const double *uu0, const double *pp00,
   else if (cache && s.phase == PH_JAC) slot = (s.sign < 0. ? 1 : 5) + s.j;
   if (slot >= 0 && !((cache->valid >> slot) & 1u)) slot = -1;
   int corr = 0, u2pret, fret = 0;
+  const unsigned in0 = s.inner[0], in1 = s.inner[1];
   if (slot >= 0) {   // evaluated ahead from the same input
     const ImpEval &e = cache->e[slot];
     for (int i = 0; i < NVR; i++) pin[i] = e.pin[i];
@@ -783,16 +821,53 @@ KG_HD int imp_advance(const RadParams &R, const double *uu0, const double *pp00,
       return IMP_OVER_CAP;
     }
     s.evals++;
-    if (s.phase == PH_BASE || s.phase == PH_JAC)
-      fret = imp_residual(R, P, pin, uu, uu0, pp00, dt, rg, u2pret, corr, f, err);
+    if (s.phase == PH_DAMP) {
+      for (int i = 0; i < NVR; i++) s.pp[i] = pin[i];   // the trial and its inversion stay in the iterate
+      const double edenmin = s.ppp[sh] / R.maxdown;
+      const double edenmax = s.ppp[sh] * R.maxup;
+      if (xxx0 > edenmin && xxx0 < edenmax && ((P.prim == IMP_MHD && corr > 0) || u2pret >= -1)) {
+        if (s.iter > R.maxiter) return imp_next_attempt(pp00, warm_guess, s, wa);
+        s.phase = PH_BASE;
+        // The base evaluation of the next iteration inverts this accepted
+        // state once more.  On MHD primitives the other component is the M1
+        // closure, a function of the conserved state alone, so it would
+        // find what is in pin, uu, u2pret and corr already: the iteration
+        // goes on from here with the residual, and counts the evaluation it
+        // does not repeat.  (Not in the entropy equation, whose residual
+        // reads uu[ENTR], nor where the base comes from the cache.)
+        if (!(P.prim == IMP_MHD && P.eq == IMP_ENERGY && !cache && budget > 0)) return IMP_RUNNING;
+        budget--;
+        s.iter++;
+        s.evals++;
+        for (int i = 0; i < NVR; i++) s.ppp[i] = s.pp[i];
+      } else {
+        if (xxx0 <= 0.) {
+          s.xiapp *= s.ppp[sh] / (s.ppp[sh] + fabs(xxx0));
+          s.xiapp *= 1.e-1;
+        } else {
+          s.xiapp /= R.dampfac;
+        }
+        if (s.xiapp < R.maxdamping) return imp_next_attempt(pp00, warm_guess, s, wa);
+        return IMP_RUNNING;
+      }
+    }
+    fret = imp_residual(R, P, pin, uu, uu0, pp00, imp_Ehat0(P, pp00, rg.g), dt, rg, u2pret, corr, f, err);
   }
   // transition
   if (s.phase == PH_BASE) {
     if (fret < 0) return imp_next_attempt(pp00, warm_guess, s, wa);
     if (err < CONV) {
       if (s.iter > R.maxiter) return imp_next_attempt(pp00, warm_guess, s, wa);   // converged past the limit (rad.c:1051)
-      s.phase = PH_FINAL;
-      return IMP_RUNNING;
+      // final inversion of the converged state (rad.c:1088-1150): it starts
+      // from the input this evaluation started from and so ends in pin; it
+      // is counted and not repeated
+      s.evals++;
+      s.inner[0] += s.inner[0] - in0;
+      s.inner[1] += s.inner[1] - in1;
+      for (int i = 0; i < NVR; i++) s.pp[i] = pin[i];
+      if ((P.prim == IMP_MHD && corr > 0) || u2pret < -1) return imp_next_attempt(pp00, warm_guess, s, wa);
+      s.pp[ENTR] = rad_Sfromu(R, s.pp[RHO], s.pp[UU]);
+      return IMP_DONE_OK;
     }
     for (int i = 0; i < 4; i++) s.f1[i] = f[i];
     s.j = 0;
@@ -800,51 +875,25 @@ KG_HD int imp_advance(const RadParams &R, const double *uu0, const double *pp00,
     s.phase = PH_JAC;
     return IMP_RUNNING;
   }
-  if (s.phase == PH_JAC) {
-    const int j = s.j;
-    if (fret < 0) {
-      if (s.sign > 0.) return imp_next_attempt(pp00, warm_guess, s, wa);
-      s.sign = 1.;
-      return IMP_RUNNING;
-    }
-    for (int i = 0; i < 4; i++) s.J[i][j] = (f[i] - s.f1[i]) / (pin[j + sh] - s.ppp[j + sh]);
-    s.j = j + 1;
-    s.sign = -1.;
-    if (s.j == 4) {
-      double iJ[4][4];
-      if (inverse_44(s.J, iJ) < 0) return imp_next_attempt(pp00, warm_guess, s, wa);
-      for (int a = 0; a < 4; a++)
-        for (int b = 0; b < 4; b++) s.J[a][b] = iJ[a][b];
-      s.xiapp = 1.;
-      s.phase = PH_DAMP;
-    }
+  // PH_JAC
+  const int j = s.j;
+  if (fret < 0) {
+    if (s.sign > 0.) return imp_next_attempt(pp00, warm_guess, s, wa);
+    s.sign = 1.;
     return IMP_RUNNING;
   }
-  if (s.phase == PH_DAMP) {
-    for (int i = 0; i < NVR; i++) s.pp[i] = pin[i];   // the trial and its inversion stay in the iterate
-    if (P.prim == IMP_MHD && corr > 0) u2pret = -1;
-    const double edenmin = s.ppp[sh] / R.maxdown;
-    const double edenmax = s.ppp[sh] * R.maxup;
-    if (xxx0 > edenmin && xxx0 < edenmax && u2pret >= -1) {
-      if (s.iter > R.maxiter) return imp_next_attempt(pp00, warm_guess, s, wa);
-      s.phase = PH_BASE;
-      return IMP_RUNNING;
-    }
-    if (xxx0 <= 0.) {
-      s.xiapp *= s.ppp[sh] / (s.ppp[sh] + fabs(xxx0));
-      s.xiapp *= 1.e-1;
-    } else {
-      s.xiapp /= R.dampfac;
-    }
-    if (s.xiapp < R.maxdamping) return imp_next_attempt(pp00, warm_guess, s, wa);
-    return IMP_RUNNING;
+  for (int i = 0; i < 4; i++) s.J[i][j] = (f[i] - s.f1[i]) / (pin[j + sh] - s.ppp[j + sh]);
+  s.j = j + 1;
+  s.sign = -1.;
+  if (s.j == 4) {
+    double iJ[4][4];
+    if (inverse_44(s.J, iJ) < 0) return imp_next_attempt(pp00, warm_guess, s, wa);
+    for (int a = 0; a < 4; a++)
+      for (int b = 0; b < 4; b++) s.J[a][b] = iJ[a][b];
+    s.xiapp = 1.;
+    s.phase = PH_DAMP;
   }
-  // final inversion of the converged state (rad.c:1088-1150)
-  for (int i = 0; i < NVR; i++) s.pp[i] = pin[i];
-  if (P.prim == IMP_MHD && corr > 0) u2pret = -2;
-  if (u2pret < -1) return imp_next_attempt(pp00, warm_guess, s, wa);
-  s.pp[ENTR] = rad_Sfromu(R, s.pp[RHO], s.pp[UU]);
-  return IMP_DONE_OK;
+  return IMP_RUNNING;
 }
 
 // ---------------------------------------------------------------------------
