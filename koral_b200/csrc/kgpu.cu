@@ -68,12 +68,46 @@ struct Box {
   int x0, y0, z0, nx, ny, nz;
   __host__ __device__ long n() const { return (long)nx * ny * nz; }
 };
+// (32-bit index arithmetic: a box holds far fewer than 2^31 cells)
 __device__ inline bool box_coord(const Box &b, long t, int &ix, int &iy, int &iz) {
-  if (t >= (long)b.nx * b.ny * b.nz) return false;
-  ix = b.x0 + (int)(t % b.nx);
-  long r = t / b.nx;
-  iy = b.y0 + (int)(r % b.ny);
-  iz = b.z0 + (int)(r / b.ny);
+  if (t >= b.n()) return false;
+  const unsigned u = (unsigned)t, r = u / (unsigned)b.nx;
+  ix = b.x0 + (int)(u - r * (unsigned)b.nx);
+  iz = (int)(r / (unsigned)b.ny);
+  iy = b.y0 + (int)(r - (unsigned)iz * (unsigned)b.ny);
+  iz += b.z0;
+  return true;
+}
+// The kernels that read the metric of their cell or face (up to 104 doubles
+// a cell) take a box in tiles: a block of 128 threads covers 32 neighbours
+// of the x-y plane (x fastest) at four successive z, one warp each.  With an
+// axisymmetric metric the four warps read the same metric lines, so three of
+// four reads hit L1 instead of L2; along z they share the stencil's planes.
+// With fewer than four planes a block covers 128 neighbours of one plane.
+struct Tile {
+  int lanes, planes;   // neighbours in the plane and planes per block
+};
+static inline Tile tile_of(const Box &b, int per_block) {
+  return b.nz >= 4 ? Tile{per_block / 4, 4} : Tile{per_block, 1};
+}
+static inline dim3 tile_grid(const Box &b, int per_block) {
+  const Tile t = tile_of(b, per_block);
+  return dim3((unsigned)(((long)b.nx * b.ny + t.lanes - 1) / t.lanes), (unsigned)((b.nz + t.planes - 1) / t.planes));
+}
+// the coordinates of element e (0 <= e < per_block) of this block's tile
+// and its index in the box, or false past the box's end
+__device__ inline bool tile_coord(const Box &b, int per_block, int e, int &ix, int &iy, int &iz, int &item) {
+  const bool four = b.nz >= 4;
+  const int lanes = four ? per_block >> 2 : per_block;
+  const int w = four ? e / lanes : 0;
+  const unsigned pl = blockIdx.x * (unsigned)lanes + (unsigned)(e - w * lanes);
+  const int z = (int)blockIdx.y * (four ? 4 : 1) + w;
+  if (pl >= (unsigned)(b.nx * b.ny) || z >= b.nz) return false;
+  const unsigned r = pl / (unsigned)b.nx;
+  ix = b.x0 + (int)(pl - r * (unsigned)b.nx);
+  iy = b.y0 + (int)r;
+  iz = b.z0 + z;
+  item = (int)(pl + (unsigned)z * (unsigned)(b.nx * b.ny));
   return true;
 }
 static inline unsigned nblocks(long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
@@ -339,9 +373,9 @@ __device__ inline void atomic_max_pos(double *addr, double v) {
 }
 
 __global__ void k_wavespeeds(Grid G, Box b) {
-  int ix, iy, iz;
+  int ix, iy, iz, item;
   double tsd = -1.;
-  if (box_coord(b, blockIdx.x * (long)blockDim.x + threadIdx.x, ix, iy, iz)) {
+  if (tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) {
     long c = cell_index(G, ix, iy, iz);
     double pp[NVR];
     load_cell(G.p, G.ncell, c, pp);
@@ -470,10 +504,8 @@ __global__ void __launch_bounds__(256) k_recon(Grid G, Box b, double *sl, double
 // floor's inversion then no longer sets the register budget of the common
 // path.
 template <int D, bool SPLIT, bool DEFER>
-__device__ __forceinline__ void face_flux(const Grid &G, const Box &b, const double *sl, const double *sr, long fi,
-                                          int side, unsigned pairmask) {
-  int ix, iy, iz;
-  box_coord(b, fi, ix, iy, iz);
+__device__ __forceinline__ void face_flux(const Grid &G, const Box &b, const double *sl, const double *sr, int ix,
+                                          int iy, int iz, long fi, int side, unsigned pairmask) {
   constexpr int nv = NVMAX;
   const int i = D == 0 ? ix : (D == 1 ? iy : iz);
   const long stride = D == 0 ? 1 : (D == 1 ? (long)G.sx : (long)G.sx * G.sy);
@@ -575,11 +607,11 @@ __device__ __forceinline__ void face_flux(const Grid &G, const Box &b, const dou
 
 template <int D, int MB = KGPU_FLUX_MIN_BLOCKS, bool SPLIT = false>
 __global__ void __launch_bounds__(128, MB) k_flux(Grid G, Box b, const double *sl, const double *sr) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const bool valid = t < 2 * b.n();
+  int ix, iy, iz, fi;
+  const bool valid = tile_coord(b, 64, threadIdx.x >> 1, ix, iy, iz, fi);
   const unsigned pairmask = __ballot_sync(0xffffffffu, valid);
   if (!valid) return;
-  face_flux<D, SPLIT, true>(G, b, sl, sr, t >> 1, (int)(t & 1), pairmask);
+  face_flux<D, SPLIT, true>(G, b, sl, sr, ix, iy, iz, fi, (int)(threadIdx.x & 1), pairmask);
 }
 
 // The faces k_flux left to the magnetic floor: a lane pair per face, all
@@ -594,7 +626,12 @@ __global__ void __launch_bounds__(128) k_flux_fix(Grid G, Box b, const double *s
   for (long base = warp * 16; base < n; base += nwarps * 16) {
     const long q = base + (lane >> 1);
     const unsigned pairmask = __ballot_sync(0xffffffffu, q < n);
-    if (q < n) face_flux<D, SPLIT, false>(G, b, sl, sr, G.fq[D][q], lane & 1, pairmask);
+    if (q < n) {
+      const int fi = G.fq[D][q];
+      int ix, iy, iz;
+      box_coord(b, fi, ix, iy, iz);
+      face_flux<D, SPLIT, false>(G, b, sl, sr, ix, iy, iz, fi, lane & 1, pairmask);
+    }
   }
 }
 
@@ -607,10 +644,9 @@ __global__ void __launch_bounds__(128) k_flux_fix(Grid G, Box b, const double *s
 // its own characteristic speeds (f_calc_fluxes_at_faces, finite.c:1379-1395).
 template <int D>
 __global__ void __launch_bounds__(128) k_flux_rad(Grid G, Box b) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const int side = (int)(t & 1);
-  int ix, iy, iz;
-  const bool valid = box_coord(b, t >> 1, ix, iy, iz);
+  const int side = (int)(threadIdx.x & 1);
+  int ix, iy, iz, fi;
+  const bool valid = tile_coord(b, 64, threadIdx.x >> 1, ix, iy, iz, fi);
   const unsigned pairmask = __ballot_sync(0xffffffffu, valid);
   if (!valid) return;
   const int i = D == 0 ? ix : (D == 1 ? iy : iz);
@@ -738,8 +774,8 @@ __global__ void k_emf(Grid G, Box b) {
 template <int MB = KGPU_UPDATE_MIN_BLOCKS>
 __global__ void __launch_bounds__(128, MB) k_update(Grid G, Box b, const double *dtp, double fac,
                                                                         double *save) {
-  int ix, iy, iz;
-  if (!box_coord(b, blockIdx.x * (long)blockDim.x + threadIdx.x, ix, iy, iz)) return;
+  int ix, iy, iz, item;
+  if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) return;
   constexpr int nv = NVMAX;
   const long c = cell_index(G, ix, iy, iz);
   const double dt = fac * dtp[0];
@@ -849,8 +885,8 @@ __global__ void __launch_bounds__(128, MB) k_update(Grid G, Box b, const double 
 // over EE0..FZ0): flux divergence plus the radiative metric source
 // gdet R^k_l Gamma^l_{jk} (f_metric_source_term_arb, physics.c:383-405).
 __global__ void __launch_bounds__(128) k_update_rad(Grid G, Box b, const double *dtp, double fac) {
-  int ix, iy, iz;
-  if (!box_coord(b, blockIdx.x * (long)blockDim.x + threadIdx.x, ix, iy, iz)) return;
+  int ix, iy, iz, item;
+  if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) return;
   const long c = cell_index(G, ix, iy, iz);
   const double dt = fac * dtp[0];
   double pp[NVR];
@@ -1024,9 +1060,8 @@ __device__ inline int u2p_run(const Grid &G, int Etype, U2PCell &x, int stop, do
 
 template <int MB = KGPU_U2P_MIN_BLOCKS>
 __global__ void __launch_bounds__(128, MB) k_u2p(Grid G, Box b, U2PQueues Q, int stop) {
-  int ix, iy, iz;
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (!box_coord(b, t, ix, iy, iz)) return;
+  int ix, iy, iz, t;
+  if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, t)) return;
   if (polar_cell(G, iy)) {
     // a corrected polar cell: only its field is inverted (u2p_solver_Bonly,
     // u2p.c:2356-2377), no floors, no fixup, conserved state as it is
@@ -1048,14 +1083,14 @@ __global__ void __launch_bounds__(128, MB) k_u2p(Grid G, Box b, U2PQueues Q, int
   int iter;
   const int r = u2p_run(G, 0, x, stop, W, iter);
   const bool paused = r == U2P_PAUSED;
-  queue_push(Q.slow, Q.n + 0, paused, (int)t);
+  queue_push(Q.slow, Q.n + 0, paused, t);
   count_lanes(&G.cnt[C_SLOW], paused);
   if (paused) {
     Q.w[x.c] = W;
     Q.it[x.c] = iter;
     return;
   }
-  u2p_energy_done(G, Q, (int)t, x, r, iter);
+  u2p_energy_done(G, Q, t, x, r, iter);
 }
 
 // Paused solves, one warp per cell (Etype 0: energy, 1: entropy).  All
@@ -1122,8 +1157,8 @@ __global__ void __launch_bounds__(128) k_u2p_entropy(Grid G, Box b, U2PQueues Q,
 // finite.c:4599-4604, stores only the first NVMHD variables, and those
 // were not averaged for this kind), so a correction is only counted.
 __global__ void __launch_bounds__(128) k_u2p_rad(Grid G, Box b) {
-  int ix, iy, iz;
-  if (!box_coord(b, blockIdx.x * (long)blockDim.x + threadIdx.x, ix, iy, iz)) return;
+  int ix, iy, iz, item;
+  if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) return;
   if (polar_cell(G, iy)) return;   // corrected polar cells: field only (u2p.c:49-101)
   const long c = cell_index(G, ix, iy, iz);
   double uu[NVR], pp[NVR];
@@ -1560,7 +1595,7 @@ bool kgpu_rad_opts_valid(const kgpu_rad_solver_opts &o);
 // against occupancy); the context picks one of each (kgpu_set_tuning,
 // kgpu_autotune).  Every variant performs the same arithmetic.
 template <int D>
-static void launch_flux(int mb, unsigned nb, cudaStream_t st, const Grid &G, Box b) {
+static void launch_flux(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b) {
   switch (mb) {
     case 5: k_flux<D, 5><<<nb, 128, 0, st>>>(G, b, nullptr, nullptr); break;
     case 6: k_flux<D, 6><<<nb, 128, 0, st>>>(G, b, nullptr, nullptr); break;
@@ -1569,7 +1604,7 @@ static void launch_flux(int mb, unsigned nb, cudaStream_t st, const Grid &G, Box
   }
 }
 template <int D>
-static void launch_flux_split(int mb, unsigned nb, cudaStream_t st, const Grid &G, Box b, const double *sl,
+static void launch_flux_split(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b, const double *sl,
                               const double *sr) {
   switch (mb) {
     case 5: k_flux<D, 5, true><<<nb, 128, 0, st>>>(G, b, sl, sr); break;
@@ -1586,7 +1621,7 @@ static void launch_flux_fix(bool split, int sms, cudaStream_t st, const Grid &G,
   if (split) k_flux_fix<D, true><<<2 * sms, 128, 0, st>>>(G, b, sl, sr);
   else k_flux_fix<D, false><<<2 * sms, 128, 0, st>>>(G, b, sl, sr);
 }
-static void launch_update(int mb, unsigned nb, cudaStream_t st, const Grid &G, Box b, const double *dtp, double fac,
+static void launch_update(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b, const double *dtp, double fac,
                           double *save) {
   switch (mb) {
     case 3: k_update<3><<<nb, 128, 0, st>>>(G, b, dtp, fac, save); break;
@@ -1594,7 +1629,7 @@ static void launch_update(int mb, unsigned nb, cudaStream_t st, const Grid &G, B
     default: k_update<4><<<nb, 128, 0, st>>>(G, b, dtp, fac, save); break;
   }
 }
-static void launch_u2p_first(int mb, unsigned nb, cudaStream_t st, const Grid &G, Box b, U2PQueues Q, int stop) {
+static void launch_u2p_first(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b, U2PQueues Q, int stop) {
   switch (mb) {
     case 4: k_u2p<4><<<nb, 128, 0, st>>>(G, b, Q, stop); break;
     case 6: k_u2p<6><<<nb, 128, 0, st>>>(G, b, Q, stop); break;
@@ -2221,7 +2256,7 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
   const int lim = G.int_order == 4 ? 2 : 1;
   int lx = G.nx > 1 ? lim : 0, ly = G.ny > 1 ? lim : 0, lz = G.nz > 1 ? lim : 0;
   Box wb{-lx, -ly, -lz, G.nx + 2 * lx, G.ny + 2 * ly, G.nz + 2 * lz};
-  { LaunchScope ls(c, K_WAVESPEEDS); k_wavespeeds<<<nblocks(wb.n(), 128), 128, 0, c->stream>>>(G, wb); }
+  { LaunchScope ls(c, K_WAVESPEEDS); k_wavespeeds<<<tile_grid(wb, 128), 128, 0, c->stream>>>(G, wb); }
   CKL("k_wavespeeds");
   int ey0 = G.ny > 1 ? -1 : 0, eny = G.ny > 1 ? G.ny + 2 : 1;
   int ez0 = G.nz > 1 ? -1 : 0, enz = G.nz > 1 ? G.nz + 2 : 1;
@@ -2237,8 +2272,8 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     {
       // the face flux and its magnetic-floor pass, timed as one
       LaunchScope ls(c, K_FLUX0);
-      if (c->flux_split) launch_flux_split<0>(c->flux_blocks, nblocks(2 * b.n(), 128), c->stream, G, b, c->fsl, c->fsr);
-      else launch_flux<0>(c->flux_blocks, nblocks(2 * b.n(), 128), c->stream, G, b);
+      if (c->flux_split) launch_flux_split<0>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b, c->fsl, c->fsr);
+      else launch_flux<0>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b);
       CKL("k_flux<0>");
       c->launches++;
       launch_flux_fix<0>(c->flux_split != 0, c->sm_count, c->stream, G, b, c->fsl, c->fsr);
@@ -2246,7 +2281,7 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     }
     if (G.rad) {
       LaunchScope ls(c, K_FLUXRAD0);
-      k_flux_rad<0><<<nblocks(2 * b.n(), 128), 128, 0, c->stream>>>(G, b);
+      k_flux_rad<0><<<tile_grid(b, 64), 128, 0, c->stream>>>(G, b);
       CKL("k_flux_rad<0>");
     }
   }
@@ -2261,8 +2296,8 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     {
       // the face flux and its magnetic-floor pass, timed as one
       LaunchScope ls(c, K_FLUX1);
-      if (c->flux_split) launch_flux_split<1>(c->flux_blocks, nblocks(2 * b.n(), 128), c->stream, G, b, c->fsl, c->fsr);
-      else launch_flux<1>(c->flux_blocks, nblocks(2 * b.n(), 128), c->stream, G, b);
+      if (c->flux_split) launch_flux_split<1>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b, c->fsl, c->fsr);
+      else launch_flux<1>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b);
       CKL("k_flux<1>");
       c->launches++;
       launch_flux_fix<1>(c->flux_split != 0, c->sm_count, c->stream, G, b, c->fsl, c->fsr);
@@ -2270,7 +2305,7 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     }
     if (G.rad) {
       LaunchScope ls(c, K_FLUXRAD1);
-      k_flux_rad<1><<<nblocks(2 * b.n(), 128), 128, 0, c->stream>>>(G, b);
+      k_flux_rad<1><<<tile_grid(b, 64), 128, 0, c->stream>>>(G, b);
       CKL("k_flux_rad<1>");
     }
   }
@@ -2285,8 +2320,8 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     {
       // the face flux and its magnetic-floor pass, timed as one
       LaunchScope ls(c, K_FLUX2);
-      if (c->flux_split) launch_flux_split<2>(c->flux_blocks, nblocks(2 * b.n(), 128), c->stream, G, b, c->fsl, c->fsr);
-      else launch_flux<2>(c->flux_blocks, nblocks(2 * b.n(), 128), c->stream, G, b);
+      if (c->flux_split) launch_flux_split<2>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b, c->fsl, c->fsr);
+      else launch_flux<2>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b);
       CKL("k_flux<2>");
       c->launches++;
       launch_flux_fix<2>(c->flux_split != 0, c->sm_count, c->stream, G, b, c->fsl, c->fsr);
@@ -2294,7 +2329,7 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     }
     if (G.rad) {
       LaunchScope ls(c, K_FLUXRAD2);
-      k_flux_rad<2><<<nblocks(2 * b.n(), 128), 128, 0, c->stream>>>(G, b);
+      k_flux_rad<2><<<tile_grid(b, 64), 128, 0, c->stream>>>(G, b);
       CKL("k_flux_rad<2>");
     }
   }
@@ -2306,10 +2341,10 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     CKL("k_emf_polar");
   }
   Box db = domain_box(G);
-  { LaunchScope ls(c, K_UPDATE); launch_update(c->update_blocks, nblocks(db.n(), 128), c->stream, G, db, dtp, fac, save); }
+  { LaunchScope ls(c, K_UPDATE); launch_update(c->update_blocks, tile_grid(db, 128), c->stream, G, db, dtp, fac, save); }
   CKL("k_update");
   if (G.rad) {
-    { LaunchScope ls(c, K_UPDATE_RAD); k_update_rad<<<nblocks(db.n(), 128), 128, 0, c->stream>>>(G, db, dtp, fac); }
+    { LaunchScope ls(c, K_UPDATE_RAD); k_update_rad<<<tile_grid(db, 128), 128, 0, c->stream>>>(G, db, dtp, fac); }
     CKL("k_update_rad");
   }
   return 0;
@@ -2319,7 +2354,7 @@ static int launch_u2p(kgpu_ctx *c, int combine) {
   Grid &G = c->G;
   Box db = domain_box(G);
   const int sweep = c->sm_count * 4;   // grid of the queue passes (grid-stride loops)
-  { LaunchScope ls(c, K_U2P); launch_u2p_first(c->u2p_blocks, nblocks(db.n(), 128), c->stream, G, db, c->u2pq, c->u2p_pass_iters); }
+  { LaunchScope ls(c, K_U2P); launch_u2p_first(c->u2p_blocks, tile_grid(db, 128), c->stream, G, db, c->u2pq, c->u2p_pass_iters); }
   CKL("k_u2p");
   { LaunchScope ls(c, K_U2P_RESUME); k_u2p_resume<<<sweep, 128, 0, c->stream>>>(G, db, c->u2pq, 0); }
   CKL("k_u2p_resume");
@@ -2328,7 +2363,7 @@ static int launch_u2p(kgpu_ctx *c, int combine) {
   { LaunchScope ls(c, K_U2P_RESUME_ENT); k_u2p_resume<<<sweep, 128, 0, c->stream>>>(G, db, c->u2pq, 1); }
   CKL("k_u2p_resume_entropy");
   if (G.rad) {
-    { LaunchScope ls(c, K_U2P_RAD); k_u2p_rad<<<nblocks(db.n(), 128), 128, 0, c->stream>>>(G, db); }
+    { LaunchScope ls(c, K_U2P_RAD); k_u2p_rad<<<tile_grid(db, 128), 128, 0, c->stream>>>(G, db); }
     CKL("k_u2p_rad");
   }
   { LaunchScope ls(c, K_FIXUP); k_fixup<<<nblocks(db.n(), 128), 128, 0, c->stream>>>(G, db, c->fixmark); }
