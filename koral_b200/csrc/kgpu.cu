@@ -96,12 +96,13 @@ static inline dim3 tile_grid(const Box &b, int per_block) {
 }
 // the coordinates of element e (0 <= e < per_block) of this block's tile
 // and its index in the box, or false past the box's end
-__device__ inline bool tile_coord(const Box &b, int per_block, int e, int &ix, int &iy, int &iz, int &item) {
+__device__ inline bool tile_coord(const Box &b, int per_block, int e, int &ix, int &iy, int &iz, int &item,
+                                  unsigned bx = blockIdx.x, unsigned by = blockIdx.y) {
   const bool four = b.nz >= 4;
   const int lanes = four ? per_block >> 2 : per_block;
   const int w = four ? e / lanes : 0;
-  const unsigned pl = blockIdx.x * (unsigned)lanes + (unsigned)(e - w * lanes);
-  const int z = (int)blockIdx.y * (four ? 4 : 1) + w;
+  const unsigned pl = bx * (unsigned)lanes + (unsigned)(e - w * lanes);
+  const int z = (int)by * (four ? 4 : 1) + w;
   if (pl >= (unsigned)(b.nx * b.ny) || z >= b.nz) return false;
   const unsigned r = pl / (unsigned)b.nx;
   ix = b.x0 + (int)(pl - r * (unsigned)b.nx);
@@ -115,12 +116,6 @@ static inline unsigned nblocks(long n, int bs) { return (unsigned)((n + bs - 1) 
 __device__ inline bool in_domain(const Grid &G, int ix, int iy, int iz) {
   return ix >= 0 && ix < G.nx && iy >= 0 && iy < G.ny && iz >= 0 && iz < G.nz;
 }
-// finite.c:2641-2666: ghost cells that touch the domain through a face only
-__device__ inline bool outside_gc(const Grid &G, int ix, int iy, int iz) {
-  bool inx = ix >= 0 && ix < G.nx, iny = iy >= 0 && iy < G.ny, inz = iz >= 0 && iz < G.nz;
-  return !((!inx && iny && inz) || (inx && !iny && inz) || (inx && iny && !inz) || (inx && iny && inz));
-}
-
 // every kernel carries the NVMAX MHD variables (kgpu_create rejects others)
 __device__ inline void load_cell(const double *arr, long ncell, long c, double *v) {
 #pragma unroll
@@ -143,109 +138,59 @@ __device__ inline void store_rad(double *arr, long ncell, long c, const double *
 // ---------------------------------------------------------------------------
 // boundary conditions (set_bc, finite.c:2752-2803; set_bc_core 2673-2748)
 // ---------------------------------------------------------------------------
-__global__ void k_bc_faces(Grid G, Box b) {
-  int ix, iy, iz;
-  if (!box_coord(b, blockIdx.x * (long)blockDim.x + threadIdx.x, ix, iy, iz)) return;
-  if (in_domain(G, ix, iy, iz) || outside_gc(G, ix, iy, iz)) return;
-  int d = (ix < 0 || ix >= G.nx) ? 0 : ((iy < 0 || iy >= G.ny) ? 1 : 2);
-  int c3[3] = {ix, iy, iz}, n3[3] = {G.nx, G.ny, G.nz};
-  int s3[3] = {ix, iy, iz};
-  const int kind = G.bc[d];
-  const int i = c3[d], n = n3[d];
+// One launch fills every ghost cell, one thread a cell.  The reference fills
+// the face ghosts from the domain, then the edges and corners from face
+// ghosts, pass after pass (one launch each, and within an edge line one cell
+// after another: 5 launches of 20 to 30 us on a 3D grid, bound by the chain
+// of each thread).  What a pass reads is, in primitives, a domain cell's
+// state with at most the sign of its normal components changed, so every
+// thread here goes back to the domain cell itself: nothing that a thread
+// reads is written by another.
+
+// The primitives of a cell at most one of whose coordinates lies outside the
+// domain: the cell's own, or what the face rule of that side gives it.  `from`
+// is the domain cell they come from.
+__device__ inline void face_prims(const Grid &G, int ix, int iy, int iz, double *pp, long &from) {
+  const int d = (ix < 0 || ix >= G.nx) ? 0 : ((iy < 0 || iy >= G.ny) ? 1 : ((iz < 0 || iz >= G.nz) ? 2 : -1));
   bool flip = false;
-  if (kind == KGPU_BC_OUTFLOW) {
-    s3[d] = i < 0 ? 0 : n - 1;
-  } else if (kind == KGPU_BC_REFLECT) {
-    s3[d] = i < 0 ? -i - 1 : 2 * n - i - 1;
-    flip = true;
-  } else {
-    if (i < 0) s3[d] = i + n;
-    if (i > n - 1) s3[d] = i - n;
-    if (d > 0 && n < G.ng) s3[d] = 0;   // finite.c:2705, 2720
+  if (d >= 0) {
+    const int kind = G.bc[d], n = d == 0 ? G.nx : (d == 1 ? G.ny : G.nz), i = d == 0 ? ix : (d == 1 ? iy : iz);
+    int src = i;
+    if (kind == KGPU_BC_OUTFLOW) {
+      src = i < 0 ? 0 : n - 1;
+    } else if (kind == KGPU_BC_REFLECT) {
+      src = i < 0 ? -i - 1 : 2 * n - i - 1;
+      flip = true;
+    } else {
+      if (i < 0) src = i + n;
+      if (i > n - 1) src = i - n;
+      if (d > 0 && n < G.ng) src = 0;   // finite.c:2705, 2720
+    }
+    if (d == 0) ix = src;
+    else if (d == 1) iy = src;
+    else iz = src;
   }
-  long c = cell_index(G, ix, iy, iz), s = cell_index(G, s3[0], s3[1], s3[2]);
-  double pp[NVR], uu[NVR];
-  load_cell(G.p, G.ncell, s, pp);
-  if (G.rad) load_rad(G.p, G.ncell, s, pp);
+  from = cell_index(G, ix, iy, iz);
+  load_cell(G.p, G.ncell, from, pp);
+  if (G.rad) load_rad(G.p, G.ncell, from, pp);
   if (flip) {
     // the component normal to the boundary: VX/B1 for x, VY/B2 for y, VZ/B3
     // for z, and the radiation frame's FX0/FY0/FZ0
-    pp[VX + d] = -pp[VX + d];
-    pp[B1 + d] = -pp[B1 + d];
-    if (G.rad) pp[FX0 + d] = -pp[FX0 + d];
-  }
-  if (kind == KGPU_BC_PERIODIC_COPY) {
-    load_cell(G.u, G.ncell, s, uu);
-    if (G.rad) load_rad(G.u, G.ncell, s, uu);
-  } else {
-    Geom g;
-    geom_centre(G, ix, iy, iz, g);
-    p2u_full(G, pp, uu, g);
-    if (G.rad) p2u_rad(pp, uu, g);
-  }
-  store_cell(G.p, G.ncell, c, pp);
-  store_cell(G.u, G.ncell, c, uu);
-  if (G.rad) {
-    store_rad(G.p, G.ncell, c, pp);
-    store_rad(G.u, G.ncell, c, uu);
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+      if (a == d) {
+        pp[VX + a] = -pp[VX + a];
+        pp[B1 + a] = -pp[B1 + a];
+        if (G.rad) pp[FX0 + a] = -pp[FX0 + a];
+      }
   }
 }
-
-// Corners of a 2D periodic domain, filled as the reference does
-// (finite.c:3075-3328): the first NG-1 cells of the two edges next to each
-// corner copy the adjacent edge ghost row/column, the diagonal cells take
-// the periodic image (written there as the mean of two equal cells).
-__device__ inline void corner2d_op(const Grid &G, int op, int &tx, int &ty, int &ax, int &ay, int &bx, int &by) {
-  const int NX = G.nx, NY = G.ny, NG = G.ng;
-  int per = 2 * NG;             // ops per corner
-  int corner = op / per, k = op % per;
-  // within a corner: k < 2(NG-1): copies (two per i); then the two diagonal cells
-  if (k < 2 * (NG - 1)) {
-    int i = k / 2, second = k % 2;
-    switch (corner) {
-      case 0:  // bottom-left
-        if (!second) { tx = -NG + i; ty = -1; ax = bx = -NG + i; ay = by = 0; }
-        else { tx = -1; ty = -NG + i; ax = bx = 0; ay = by = -NG + i; }
-        break;
-      case 1:  // top-left
-        if (!second) { tx = -NG + i; ty = NY; ax = bx = -NG + i; ay = by = NY - 1; }
-        else { tx = -1; ty = NY + i + 1; ax = bx = 0; ay = by = NY + i + 1; }
-        break;
-      case 2:  // bottom-right
-        if (!second) { tx = NX + i + 1; ty = -1; ax = bx = NX + i + 1; ay = by = 0; }
-        else { tx = NX; ty = -NG + i; ax = bx = NX - 1; ay = by = -NG + i; }
-        break;
-      default:  // top-right
-        if (!second) { tx = NX + i + 1; ty = NY; ax = bx = NX + i + 1; ay = by = NY - 1; }
-        else { tx = NX; ty = NY + i + 1; ax = bx = NX - 1; ay = by = NY + i + 1; }
-        break;
-    }
-    return;
-  }
-  int j = k - 2 * (NG - 1);    // 0: first diagonal cell, 1: second
-  switch (corner) {
-    case 0: tx = -1 - j; ty = -1 - j; ax = bx = NX - 1 - j; ay = by = -1 - j; break;
-    case 1: tx = -1 - j; ty = NY + j; ax = bx = NX - 1 - j; ay = by = NY + j; break;
-    case 2: tx = NX + j; ty = -1 - j; ax = bx = 0 + j; ay = by = -1 - j; break;
-    default: tx = NX + j; ty = NY + j; ax = bx = 0 + j; ay = by = NY + j; break;
-  }
-}
-__global__ void k_bc_corners2d(Grid G) {
-  int op = blockIdx.x * blockDim.x + threadIdx.x;
-  if (op >= 8 * G.ng) return;
-  int tx, ty, ax, ay, bx, by;
-  corner2d_op(G, op, tx, ty, ax, ay, bx, by);
-  int k = op % (2 * G.ng);
-  bool avg = k >= 2 * (G.ng - 1);
-  long ca = cell_index(G, ax, ay, 0), cb = cell_index(G, bx, by, 0), c = cell_index(G, tx, ty, 0);
-  double pp[NVR], uu[NVR];
-  const int nv = G.rad ? NVR : NVMAX;
-  for (int iv = 0; iv < nv; iv++) {
-    double a = G.p[iv * G.ncell + ca];
-    pp[iv] = avg ? .5 * (a + G.p[iv * G.ncell + cb]) : a;
-  }
+// the ghost cell (ix, iy, iz) from primitives pp; uu from p2u
+__device__ inline void ghost_store(const Grid &G, int ix, int iy, int iz, const double *pp) {
+  const long c = cell_index(G, ix, iy, iz);
+  double uu[NVR];
   Geom g;
-  geom_centre(G, tx, ty, 0, g);
+  geom_centre(G, ix, iy, iz, g);
   p2u_full(G, pp, uu, g);
   store_cell(G.p, G.ncell, c, pp);
   store_cell(G.u, G.ncell, c, uu);
@@ -256,50 +201,14 @@ __global__ void k_bc_corners2d(Grid G) {
   }
 }
 
-// Edges and corners of a 3D domain with physical boundaries, in the
-// reference's order (finite.c:3330-3705): edges elongated along z, then
-// along y, then along x, each filling the first NG-1 cells of the two faces
-// next to the edge from the adjacent ghost row and two diagonal cells as
-// means of their neighbours; then the eight NG^3 corner blocks copy the
-// nearest domain corner cell.  A pass reads only cells that earlier passes
-// (or the face fill) wrote, so the lines of one pass run in parallel.
-__device__ inline void set_from(const Grid &G, int tx, int ty, int tz, int s1x, int s1y, int s1z, int s2x, int s2y,
-                                int s2z, bool avg) {
-  long c = cell_index(G, tx, ty, tz), a = cell_index(G, s1x, s1y, s1z), b = cell_index(G, s2x, s2y, s2z);
-  double pp[NVR], uu[NVR];
-  const int nv = G.rad ? NVR : NVMAX;
-  for (int iv = 0; iv < nv; iv++) {
-    double va = G.p[iv * G.ncell + a];
-    pp[iv] = avg ? .5 * (va + G.p[iv * G.ncell + b]) : va;
-  }
-  Geom g;
-  geom_centre(G, tx, ty, tz, g);
-  p2u_full(G, pp, uu, g);
-  store_cell(G.p, G.ncell, c, pp);
-  store_cell(G.u, G.ncell, c, uu);
-  if (G.rad) {
-    p2u_rad(pp, uu, g);
-    store_rad(G.p, G.ncell, c, pp);
-    store_rad(G.u, G.ncell, c, uu);
-  }
-}
-// one line of one elongated-edge pass.  Edge axis c, the two other axes
-// (a, b); corner k: bit 1 = high end of a, bit 0 = high end of b; position t
-// along c in [-NG, N_c+NG).  In (a, b) coordinates, with the ghost layers
-// counted outwards, the reference writes for i = 0..NG-2
+// Cells of an edge of the domain, axes (a, b) across it, corner k (bit 1:
+// high end of a, bit 0: high end of b).  In (a, b), with the ghost layers
+// counted outwards, the reference (2D: finite.c:3075-3328; 3D edges:
+// 3330-3705) writes for i = 0..NG-2
 //   lo,lo: (-NG+i,-1)<-(-NG+i,0)      (-1,-NG+i)<-(0,-NG+i)
 //   lo,hi: (-NG+i,NB)<-(-NG+i,NB-1)   (-1,NB+i+1)<-(0,NB+i+1)
 //   hi,lo: (NA,-NG+i)<-(NA-1,-NG+i)   (NA+i+1,-1)<-(NA+i+1,0)
 //   hi,hi: (NA+i+1,NB)<-(NA+i+1,NB-1) (NA,NB+i+1)<-(NA-1,NB+i+1)
-// and then the two diagonal cells as means of their inner neighbours.
-// (x, y, z) of the cell at (va, vb) in the (a, b) plane and t along c;
-// plain selects, no indexed local array
-__device__ inline void at3(int c, int a, int b, int t, int va, int vb, int &x, int &y, int &z) {
-  x = a == 0 ? va : (b == 0 ? vb : t);
-  y = a == 1 ? va : (b == 1 ? vb : t);
-  z = a == 2 ? va : (b == 2 ? vb : t);
-  (void)c;
-}
 // target (ta, tb) and source (sa, sb) of copy j of ghost layer i
 __device__ inline void edge_copy(bool hiA, bool hiB, int NG, int NA, int NB, int i, int j, int &ta, int &tb, int &sa,
                                  int &sb) {
@@ -317,50 +226,135 @@ __device__ inline void edge_copy(bool hiA, bool hiB, int NG, int NA, int NB, int
     else { ta = NA; tb = NB + i + 1; sa = NA - 1; sb = NB + i + 1; }
   }
 }
-__global__ void k_bc_edges3d(Grid G, int c, int a, int b) {
-  const int NG = G.ng;
-  const int NA = a == 0 ? G.nx : (a == 1 ? G.ny : G.nz);
-  const int NB = b == 0 ? G.nx : (b == 1 ? G.ny : G.nz);
-  const int NC = c == 0 ? G.nx : (c == 1 ? G.ny : G.nz);
-  int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  int len = NC + 2 * NG;
-  if (tid >= 4 * len) return;
-  const int k = tid / len, t = tid % len - NG;
-  const bool hiA = (k >> 1) & 1, hiB = k & 1;
-  int x, y, z, x1, y1, z1, x2, y2, z2;
-  for (int i = 0; i < NG - 1; i++)
-    for (int j = 0; j < 2; j++) {
-      int ta, tb, sa, sb;
-      edge_copy(hiA, hiB, NG, NA, NB, i, j, ta, tb, sa, sb);
-      at3(c, a, b, t, ta, tb, x, y, z);
-      at3(c, a, b, t, sa, sb, x1, y1, z1);
-      set_from(G, x, y, z, x1, y1, z1, x1, y1, z1, false);
-    }
-  // diagonal cells: g1 = first ghost layer in both a and b, g2 = second;
-  // mean of (g.a, g.b - sB) and (g.a - sA, g.b), s pointing out of the domain
-  const int sA = hiA ? 1 : -1, sB = hiB ? 1 : -1;
-  const int g1a = hiA ? NA : -1, g1b = hiB ? NB : -1;
-  at3(c, a, b, t, g1a, g1b, x, y, z);
-  at3(c, a, b, t, g1a, g1b - sB, x1, y1, z1);
-  at3(c, a, b, t, g1a - sA, g1b, x2, y2, z2);
-  set_from(G, x, y, z, x1, y1, z1, x2, y2, z2, true);
-  const int g2a = g1a + sA, g2b = g1b + sB;
-  at3(c, a, b, t, g2a, g2b, x, y, z);
-  at3(c, a, b, t, g2a, g2b - sB, x1, y1, z1);
-  at3(c, a, b, t, g2a - sA, g2b, x2, y2, z2);
-  set_from(G, x, y, z, x1, y1, z1, x2, y2, z2, true);
+// (x, y, z) of the cell at (va, vb) in the (a, b) plane and t along c;
+// plain selects, no indexed local array
+__device__ inline void at3(int a, int b, int t, int va, int vb, int &x, int &y, int &z) {
+  x = a == 0 ? va : (b == 0 ? vb : t);
+  y = a == 1 ? va : (b == 1 ? vb : t);
+  z = a == 2 ? va : (b == 2 ? vb : t);
 }
-__global__ void k_bc_corners3d(Grid G) {
+
+// threads of k_bc by part: the ghost slabs of the three faces, the edges
+// elongated along z, y and x (2 NG cells of each position of each line: the
+// copies, then the two diagonal cells as means of two neighbours), and the
+// corner blocks (3D).  The edge positions in the ghost range of their own
+// axis are corner cells, which the reference overwrites with the corner
+// blocks.
+struct BcParts {
+  int n[7];   // number of threads of each part: faces x, y, z; edges z, y, x; corners
+  __host__ __device__ int total() const {
+    int t = 0;
+    for (int k = 0; k < 7; k++) t += n[k];
+    return t;
+  }
+};
+static BcParts bc_parts(const Grid &G) {
+  BcParts P{};
   const int NG = G.ng;
-  int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  int per = NG * NG * NG;
-  if (tid >= 8 * per) return;
-  int k = tid / per, r = tid % per;
-  bool hx = k & 1, hy = (k >> 1) & 1, hz = (k >> 2) & 1;
-  int ox = r % NG, oy = (r / NG) % NG, oz = r / (NG * NG);
-  int tx = hx ? G.nx + ox : -NG + ox, ty = hy ? G.ny + oy : -NG + oy, tz = hz ? G.nz + oz : -NG + oz;
-  int sx = hx ? G.nx - 1 : 0, sy = hy ? G.ny - 1 : 0, sz = hz ? G.nz - 1 : 0;
-  set_from(G, tx, ty, tz, sx, sy, sz, sx, sy, sz, false);
+  P.n[0] = 2 * G.ngcx * G.ny * G.nz;
+  P.n[1] = 2 * G.ngcy * G.nx * G.nz;
+  P.n[2] = 2 * G.ngcz * G.nx * G.ny;
+  if (G.ny > 1) P.n[3] = 4 * 2 * NG * G.nz;
+  if (G.ny > 1 && G.nz > 1) {
+    P.n[4] = 4 * 2 * NG * G.ny;
+    P.n[5] = 4 * 2 * NG * G.nx;
+    P.n[6] = 8 * NG * NG * NG;
+  }
+  return P;
+}
+
+__global__ void __launch_bounds__(128) k_bc(Grid G, BcParts P) {
+  int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  int part = 0;
+  while (part < 7 && t >= P.n[part]) t -= P.n[part++];
+  if (part == 7) return;
+  const int NG = G.ng;
+  double pp[NVR];
+  long from;
+  if (part < 3) {
+    // ghost layer m of the slab: -NG..-1, then n..n+NG-1
+    int ix, iy, iz, m;
+    if (part == 0) {
+      m = t % (2 * NG); t /= 2 * NG;
+      iy = t % G.ny; iz = t / G.ny;
+      ix = m < NG ? m - NG : G.nx + m - NG;
+    } else if (part == 1) {
+      ix = t % G.nx; t /= G.nx;
+      m = t % (2 * NG); iz = t / (2 * NG);
+      iy = m < NG ? m - NG : G.ny + m - NG;
+    } else {
+      ix = t % G.nx; t /= G.nx;
+      iy = t % G.ny; m = t / G.ny;
+      iz = m < NG ? m - NG : G.nz + m - NG;
+    }
+    face_prims(G, ix, iy, iz, pp, from);
+    if (G.bc[part] == KGPU_BC_PERIODIC_COPY) {
+      const long c = cell_index(G, ix, iy, iz);
+      double uu[NVR];
+      load_cell(G.u, G.ncell, from, uu);
+      store_cell(G.p, G.ncell, c, pp);
+      store_cell(G.u, G.ncell, c, uu);
+      if (G.rad) {
+        load_rad(G.u, G.ncell, from, uu);
+        store_rad(G.p, G.ncell, c, pp);
+        store_rad(G.u, G.ncell, c, uu);
+      }
+    } else {
+      ghost_store(G, ix, iy, iz, pp);
+    }
+    return;
+  }
+  if (part == 6) {
+    const int per = NG * NG * NG, k = t / per, r = t % per;
+    const bool hx = k & 1, hy = (k >> 1) & 1, hz = (k >> 2) & 1;
+    const int ox = r % NG, oy = (r / NG) % NG, oz = r / (NG * NG);
+    face_prims(G, hx ? G.nx - 1 : 0, hy ? G.ny - 1 : 0, hz ? G.nz - 1 : 0, pp, from);
+    ghost_store(G, hx ? G.nx + ox : -NG + ox, hy ? G.ny + oy : -NG + oy, hz ? G.nz + oz : -NG + oz, pp);
+    return;
+  }
+  // edges along z (a = x, b = y), along y (a = x, b = z), along x (a = y, b = z)
+  const int a = part == 5 ? 1 : 0, b = part == 3 ? 1 : 2;
+  const int NA = a == 0 ? G.nx : G.ny, NB = b == 1 ? G.ny : G.nz, NC = part == 3 ? G.nz : (part == 4 ? G.ny : G.nx);
+  const int pos = t % NC;   // along the edge
+  t /= NC;
+  const int k = t / (2 * NG), op = t % (2 * NG);
+  const bool hiA = (k >> 1) & 1, hiB = k & 1;
+  int x, y, z, x1, y1, z1;
+  if (op < 2 * (NG - 1)) {
+    int ta, tb, sa, sb;
+    edge_copy(hiA, hiB, NG, NA, NB, op / 2, op % 2, ta, tb, sa, sb);
+    at3(a, b, pos, ta, tb, x, y, z);
+    at3(a, b, pos, sa, sb, x1, y1, z1);
+    face_prims(G, x1, y1, z1, pp, from);
+  } else {
+    // diagonal cell j: the first from the two face ghosts beside it, the
+    // second from the copies beside it, whose primitives are those of the
+    // face ghosts they were made from (the same cells of the next layer)
+    const int j = op - 2 * (NG - 1);
+    const int sA = hiA ? 1 : -1, sB = hiB ? 1 : -1;
+    const int ga = (hiA ? NA : -1) + j * sA, gb = (hiB ? NB : -1) + j * sB;
+    const int ina = hiA ? NA - 1 : 0, inb = hiB ? NB - 1 : 0;
+    at3(a, b, pos, ga, gb, x, y, z);
+    if (G.nz == 1) {
+      // 2D periodic corners: the mean of two equal cells, the periodic image
+      // along x of the row outside (finite.c:3075-3328)
+      at3(a, b, pos, hiA ? j : NA - 1 - j, gb, x1, y1, z1);
+      face_prims(G, x1, y1, z1, pp, from);
+#pragma unroll
+      for (int iv = 0; iv < NVR; iv++)
+        if (iv < NVMAX || G.rad) pp[iv] = .5 * (pp[iv] + pp[iv]);
+    } else {
+      double p2[NVR];
+      at3(a, b, pos, ga, inb, x1, y1, z1);
+      face_prims(G, x1, y1, z1, pp, from);
+      at3(a, b, pos, ina, gb, x1, y1, z1);
+      face_prims(G, x1, y1, z1, p2, from);
+#pragma unroll
+      for (int iv = 0; iv < NVR; iv++)
+        if (iv < NVMAX || G.rad) pp[iv] = .5 * (pp[iv] + p2[iv]);
+    }
+  }
+  ghost_store(G, x, y, z, pp);
 }
 
 // ---------------------------------------------------------------------------
@@ -373,6 +367,7 @@ __device__ inline void atomic_max_pos(double *addr, double v) {
 }
 
 __global__ void k_wavespeeds(Grid G, Box b) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 3) G.fqn[threadIdx.x] = 0;   // the flux kernels' queues
   int ix, iy, iz, item;
   double tsd = -1.;
   if (tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) {
@@ -614,10 +609,34 @@ __global__ void __launch_bounds__(128, MB) k_flux(Grid G, Box b, const double *s
   face_flux<D, SPLIT, true>(G, b, sl, sr, ix, iy, iz, fi, (int)(threadIdx.x & 1), pairmask);
 }
 
+// The three directions in one launch, for grids too small to fill the chip
+// with one of them: blocks [0, n0) take the x faces, the next n1 the y faces,
+// the rest the z faces.  Compiled for four blocks per SM (128 registers, next
+// to no spills): with so few blocks a thread's chain counts, not occupancy.
+struct FaceBoxes {
+  Box b[3];
+  unsigned gx[3], n[3];   // tiles of the plane; blocks
+};
+__global__ void __launch_bounds__(128, 4) k_flux_all(Grid G, FaceBoxes F) {
+  const unsigned t0 = blockIdx.x;
+  const int d = t0 < F.n[0] ? 0 : (t0 < F.n[0] + F.n[1] ? 1 : 2);
+  const unsigned t = t0 - (d > 0 ? F.n[0] : 0u) - (d > 1 ? F.n[1] : 0u);
+  const unsigned gx = d == 0 ? F.gx[0] : (d == 1 ? F.gx[1] : F.gx[2]);
+  const Box b = d == 0 ? F.b[0] : (d == 1 ? F.b[1] : F.b[2]);
+  int ix, iy, iz, fi;
+  const bool valid = tile_coord(b, 64, threadIdx.x >> 1, ix, iy, iz, fi, t % gx, t / gx);
+  const unsigned pairmask = __ballot_sync(0xffffffffu, valid);
+  if (!valid) return;
+  const int side = (int)(threadIdx.x & 1);
+  if (d == 0) face_flux<0, false, true>(G, b, nullptr, nullptr, ix, iy, iz, fi, side, pairmask);
+  else if (d == 1) face_flux<1, false, true>(G, b, nullptr, nullptr, ix, iy, iz, fi, side, pairmask);
+  else face_flux<2, false, true>(G, b, nullptr, nullptr, ix, iy, iz, fi, side, pairmask);
+}
+
 // The faces k_flux left to the magnetic floor: a lane pair per face, all
 // registers the floor's inversion wants.  The loop runs warp-uniformly.
 template <int D, bool SPLIT>
-__global__ void __launch_bounds__(128) k_flux_fix(Grid G, Box b, const double *sl, const double *sr) {
+__device__ __forceinline__ void flux_fix(const Grid &G, const Box &b, const double *sl, const double *sr) {
   const int n = *(volatile int *)(G.fqn + D);
   if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(G.cnt + C_FACE_FLOOR, (unsigned long long)n);
   const long warp = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
@@ -634,6 +653,17 @@ __global__ void __launch_bounds__(128) k_flux_fix(Grid G, Box b, const double *s
     }
   }
 }
+// one direction (the split form reuses its face states for the next one)
+template <int D>
+__global__ void __launch_bounds__(128) k_flux_fix(Grid G, Box b, const double *sl, const double *sr) {
+  flux_fix<D, true>(G, b, sl, sr);
+}
+// all directions, their queues one after another: empty on most steps
+__global__ void __launch_bounds__(128) k_flux_fix_all(Grid G, FaceBoxes F) {
+  if (F.n[0]) flux_fix<0, false>(G, F.b[0], nullptr, nullptr);
+  if (F.n[1]) flux_fix<1, false>(G, F.b[1], nullptr, nullptr);
+  if (F.n[2]) flux_fix<2, false>(G, F.b[2], nullptr, nullptr);
+}
 
 // Radiative face fluxes (the EE0..FZ0 part of the same face loop): the
 // reference reconstructs all thirteen variables together, but nothing of
@@ -643,12 +673,7 @@ __global__ void __launch_bounds__(128) k_flux_fix(Grid G, Box b, const double *s
 // the radiation runs as its own kernel with the same two-lane layout and
 // its own characteristic speeds (f_calc_fluxes_at_faces, finite.c:1379-1395).
 template <int D>
-__global__ void __launch_bounds__(128) k_flux_rad(Grid G, Box b) {
-  const int side = (int)(threadIdx.x & 1);
-  int ix, iy, iz, fi;
-  const bool valid = tile_coord(b, 64, threadIdx.x >> 1, ix, iy, iz, fi);
-  const unsigned pairmask = __ballot_sync(0xffffffffu, valid);
-  if (!valid) return;
+__device__ __forceinline__ void face_flux_rad(const Grid &G, int ix, int iy, int iz, int side, unsigned pairmask) {
   const int i = D == 0 ? ix : (D == 1 ? iy : iz);
   const long stride = D == 0 ? 1 : (D == 1 ? (long)G.sx : (long)G.sx * G.sy);
   const long cR = cell_index(G, ix, iy, iz);
@@ -707,6 +732,30 @@ __global__ void __launch_bounds__(128) k_flux_rad(Grid G, Box b) {
     }
     out[(EE0 + j) * nf] = fl;
   }
+}
+
+template <int D>
+__global__ void __launch_bounds__(128) k_flux_rad(Grid G, Box b) {
+  int ix, iy, iz, fi;
+  const bool valid = tile_coord(b, 64, threadIdx.x >> 1, ix, iy, iz, fi);
+  const unsigned pairmask = __ballot_sync(0xffffffffu, valid);
+  if (valid) face_flux_rad<D>(G, ix, iy, iz, (int)(threadIdx.x & 1), pairmask);
+}
+// the three directions in one launch, as k_flux_all
+__global__ void __launch_bounds__(128) k_flux_rad_all(Grid G, FaceBoxes F) {
+  const unsigned t0 = blockIdx.x;
+  const int d = t0 < F.n[0] ? 0 : (t0 < F.n[0] + F.n[1] ? 1 : 2);
+  const unsigned t = t0 - (d > 0 ? F.n[0] : 0u) - (d > 1 ? F.n[1] : 0u);
+  const unsigned gx = d == 0 ? F.gx[0] : (d == 1 ? F.gx[1] : F.gx[2]);
+  const Box b = d == 0 ? F.b[0] : (d == 1 ? F.b[1] : F.b[2]);
+  int ix, iy, iz, fi;
+  const bool valid = tile_coord(b, 64, threadIdx.x >> 1, ix, iy, iz, fi, t % gx, t / gx);
+  const unsigned pairmask = __ballot_sync(0xffffffffu, valid);
+  if (!valid) return;
+  const int side = (int)(threadIdx.x & 1);
+  if (d == 0) face_flux_rad<0>(G, ix, iy, iz, side, pairmask);
+  else if (d == 1) face_flux_rad<1>(G, ix, iy, iz, side, pairmask);
+  else face_flux_rad<2>(G, ix, iy, iz, side, pairmask);
 }
 
 // zero fluxes outside the Riemann range (finite.c:1520, 1620): only needed
@@ -1573,14 +1622,14 @@ __global__ void k_fill(double *a, long n, double v) {
 enum KernelId { K_BC = 0, K_WAVESPEEDS, K_FLUX0, K_FLUX1, K_FLUX2, K_EMF, K_UPDATE, K_U2P, K_U2P_RESUME,
                 K_U2P_ENT, K_U2P_RESUME_ENT, K_FIXUP, K_COMMIT, K_BEGIN, K_FLUXRAD0, K_FLUXRAD1, K_FLUXRAD2,
                 K_UPDATE_RAD, K_U2P_RAD, K_IMP_GATHER, K_IMP_WARM, K_IMP_SOLVE, K_IMP_SCATTER, K_IMEX, K_RECON0,
-                K_RECON1, K_RECON2, K_AVG, K_NKERNELS };
+                K_RECON1, K_RECON2, K_AVG, K_FLUX_FIX, K_NKERNELS };
 static const char *kKernelNames[K_NKERNELS] = {"k_bc", "k_wavespeeds", "k_flux_x", "k_flux_y", "k_flux_z", "k_emf",
                                                "k_update", "k_u2p", "k_u2p_resume", "k_u2p_entropy",
                                                "k_u2p_resume_entropy", "k_fixup", "k_commit", "k_begin_step",
                                                "k_flux_rad_x", "k_flux_rad_y", "k_flux_rad_z", "k_update_rad",
                                                "k_u2p_rad", "k_imp_gather", "k_imp_warm_start", "k_imp_solve",
                                                "k_imp_scatter", "k_imex", "k_recon_x", "k_recon_y", "k_recon_z",
-                                               "k_save_avg"};
+                                               "k_save_avg", "k_flux_fix"};
 
 int kgpu_rad_solve_enqueue(int n, const kgpu_rad_params *rp, const double *uu, const double *pp, const double *g,
                            const double *G, const double *dt, const float *ypred, double *pp_out, double *uu_out,
@@ -1612,14 +1661,6 @@ static void launch_flux_split(int mb, dim3 nb, cudaStream_t st, const Grid &G, B
     case 8: k_flux<D, 8, true><<<nb, 128, 0, st>>>(G, b, sl, sr); break;
     default: k_flux<D, 7, true><<<nb, 128, 0, st>>>(G, b, sl, sr); break;
   }
-}
-// the faces of direction D that k_flux left to the magnetic floor: two
-// blocks per SM loop over the queue (empty on most steps)
-template <int D>
-static void launch_flux_fix(bool split, int sms, cudaStream_t st, const Grid &G, Box b, const double *sl,
-                            const double *sr) {
-  if (split) k_flux_fix<D, true><<<2 * sms, 128, 0, st>>>(G, b, sl, sr);
-  else k_flux_fix<D, false><<<2 * sms, 128, 0, st>>>(G, b, sl, sr);
 }
 static void launch_update(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b, const double *dtp, double fac,
                           double *save) {
@@ -2224,29 +2265,9 @@ extern "C" int kgpu_read_restart(kgpu_ctx *c, const char *folder, int nout1, dou
 
 static int launch_bc(kgpu_ctx *c) {
   Grid &G = c->G;
-  Box b{-G.ngcx, -G.ngcy, -G.ngcz, G.sx, G.sy, G.sz};
-  { LaunchScope ls(c, K_BC); k_bc_faces<<<nblocks(b.n(), 128), 128, 0, c->stream>>>(G, b); }
-  CKL("k_bc_faces");
-  if (G.nz == 1 && G.ny > 1) {
-    LaunchScope ls(c, K_BC);
-    k_bc_corners2d<<<1, 8 * G.ng > 32 ? 64 : 32, 0, c->stream>>>(G);
-    CKL("k_bc_corners2d");
-  }
-  if (G.nz > 1 && G.ny > 1) {
-    // edges along z (a=x, b=y), along y (a=x, b=z), along x (a=y, b=z)
-    const int axes[3][3] = {{2, 0, 1}, {1, 0, 2}, {0, 1, 2}};
-    int n3[3] = {G.nx, G.ny, G.nz};
-    for (int k = 0; k < 3; k++) {
-      int cax = axes[k][0];
-      int nthreads = 4 * (n3[cax] + 2 * G.ng);
-      LaunchScope ls(c, K_BC);
-      k_bc_edges3d<<<nblocks(nthreads, 128), 128, 0, c->stream>>>(G, cax, axes[k][1], axes[k][2]);
-      CKL("k_bc_edges3d");
-    }
-    LaunchScope ls(c, K_BC);
-    k_bc_corners3d<<<nblocks(8 * G.ng * G.ng * G.ng, 128), 128, 0, c->stream>>>(G);
-    CKL("k_bc_corners3d");
-  }
+  const BcParts P = bc_parts(G);
+  { LaunchScope ls(c, K_BC); k_bc<<<nblocks(P.total(), 128), 128, 0, c->stream>>>(G, P); }
+  CKL("k_bc");
   return 0;
 }
 
@@ -2261,77 +2282,65 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
   int ey0 = G.ny > 1 ? -1 : 0, eny = G.ny > 1 ? G.ny + 2 : 1;
   int ez0 = G.nz > 1 ? -1 : 0, enz = G.nz > 1 ? G.nz + 2 : 1;
   int ex0 = -1, enx = G.nx + 2;
-  if (G.nx > 1) {
-    Box b{0, ey0, ez0, G.nx + 1, eny, enz};
-    CK(cudaMemsetAsync(G.fqn + 0, 0, sizeof(int), c->stream));
-    if (c->flux_split) {
-      { LaunchScope ls(c, K_RECON0);
-        k_recon<0><<<nblocks(b.n() * NVMAX, 256), 256, 0, c->stream>>>(G, b, c->fsl, c->fsr); }
-      CKL("k_recon<0>");
-    }
-    {
-      // the face flux and its magnetic-floor pass, timed as one
-      LaunchScope ls(c, K_FLUX0);
-      if (c->flux_split) launch_flux_split<0>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b, c->fsl, c->fsr);
-      else launch_flux<0>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b);
-      CKL("k_flux<0>");
-      c->launches++;
-      launch_flux_fix<0>(c->flux_split != 0, c->sm_count, c->stream, G, b, c->fsl, c->fsr);
-      CKL("k_flux_fix<0>");
-    }
-    if (G.rad) {
-      LaunchScope ls(c, K_FLUXRAD0);
-      k_flux_rad<0><<<tile_grid(b, 64), 128, 0, c->stream>>>(G, b);
-      CKL("k_flux_rad<0>");
-    }
+  FaceBoxes F{};
+  F.b[0] = Box{0, ey0, ez0, G.nx > 1 ? G.nx + 1 : 0, eny, enz};
+  F.b[1] = Box{ex0, 0, ez0, enx, G.ny > 1 ? G.ny + 1 : 0, enz};
+  F.b[2] = Box{ex0, ey0, 0, enx, eny, G.nz > 1 ? G.nz + 1 : 0};
+  for (int d = 0; d < 3; d++) {
+    if (F.b[d].n() == 0) continue;
+    const dim3 g = tile_grid(F.b[d], 64);
+    F.gx[d] = g.x;
+    F.n[d] = g.x * g.y;
   }
-  if (G.ny > 1) {
-    Box b{ex0, 0, ez0, enx, G.ny + 1, enz};
-    CK(cudaMemsetAsync(G.fqn + 1, 0, sizeof(int), c->stream));
-    if (c->flux_split) {
-      { LaunchScope ls(c, K_RECON1);
-        k_recon<1><<<nblocks(b.n() * NVMAX, 256), 256, 0, c->stream>>>(G, b, c->fsl, c->fsr); }
-      CKL("k_recon<1>");
-    }
-    {
-      // the face flux and its magnetic-floor pass, timed as one
-      LaunchScope ls(c, K_FLUX1);
-      if (c->flux_split) launch_flux_split<1>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b, c->fsl, c->fsr);
-      else launch_flux<1>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b);
-      CKL("k_flux<1>");
-      c->launches++;
-      launch_flux_fix<1>(c->flux_split != 0, c->sm_count, c->stream, G, b, c->fsl, c->fsr);
-      CKL("k_flux_fix<1>");
-    }
+  const unsigned nall = F.n[0] + F.n[1] + F.n[2];
+  // One launch for the three directions while they fill the chip only a few
+  // times: on the 128x128 vortex, 268 blocks a direction, a launch takes as
+  // long as one thread's chain whatever it computes.  Larger grids lose
+  // nothing to the launches and gain from k_flux's occupancy.  A profiled step
+  // shows the directions apart.
+  const bool together = !c->flux_split && !c->profiling && nall <= 16u * (unsigned)c->sm_count;
+  if (together) {
+    { LaunchScope ls(c, K_FLUX0); k_flux_all<<<nall, 128, 0, c->stream>>>(G, F); }
+    CKL("k_flux_all");
     if (G.rad) {
-      LaunchScope ls(c, K_FLUXRAD1);
-      k_flux_rad<1><<<tile_grid(b, 64), 128, 0, c->stream>>>(G, b);
-      CKL("k_flux_rad<1>");
+      { LaunchScope ls(c, K_FLUXRAD0); k_flux_rad_all<<<nall, 128, 0, c->stream>>>(G, F); }
+      CKL("k_flux_rad_all");
     }
+  } else {
+#define FLUX_DIR(D)                                                                                                   \
+  if (F.n[D]) {                                                                                                       \
+    const Box b = F.b[D];                                                                                             \
+    if (c->flux_split) {                                                                                              \
+      { LaunchScope ls(c, K_RECON0 + D);                                                                              \
+        k_recon<D><<<nblocks(b.n() * NVMAX, 256), 256, 0, c->stream>>>(G, b, c->fsl, c->fsr); }                        \
+      CKL("k_recon");                                                                                                 \
+      LaunchScope ls(c, K_FLUX0 + D);                                                                                 \
+      launch_flux_split<D>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b, c->fsl, c->fsr);                         \
+      CKL("k_flux");                                                                                                  \
+      c->launches++;                                                                                                  \
+      k_flux_fix<D><<<2 * c->sm_count, 128, 0, c->stream>>>(G, b, c->fsl, c->fsr);                                     \
+      CKL("k_flux_fix");                                                                                              \
+    } else {                                                                                                          \
+      LaunchScope ls(c, K_FLUX0 + D);                                                                                 \
+      launch_flux<D>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b);                                               \
+      CKL("k_flux");                                                                                                  \
+    }                                                                                                                 \
+    if (G.rad) {                                                                                                      \
+      LaunchScope ls(c, K_FLUXRAD0 + D);                                                                              \
+      k_flux_rad<D><<<tile_grid(b, 64), 128, 0, c->stream>>>(G, b);                                                    \
+      CKL("k_flux_rad");                                                                                              \
+    }                                                                                                                 \
   }
-  if (G.nz > 1) {
-    Box b{ex0, ey0, 0, enx, eny, G.nz + 1};
-    CK(cudaMemsetAsync(G.fqn + 2, 0, sizeof(int), c->stream));
-    if (c->flux_split) {
-      { LaunchScope ls(c, K_RECON2);
-        k_recon<2><<<nblocks(b.n() * NVMAX, 256), 256, 0, c->stream>>>(G, b, c->fsl, c->fsr); }
-      CKL("k_recon<2>");
-    }
-    {
-      // the face flux and its magnetic-floor pass, timed as one
-      LaunchScope ls(c, K_FLUX2);
-      if (c->flux_split) launch_flux_split<2>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b, c->fsl, c->fsr);
-      else launch_flux<2>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b);
-      CKL("k_flux<2>");
-      c->launches++;
-      launch_flux_fix<2>(c->flux_split != 0, c->sm_count, c->stream, G, b, c->fsl, c->fsr);
-      CKL("k_flux_fix<2>");
-    }
-    if (G.rad) {
-      LaunchScope ls(c, K_FLUXRAD2);
-      k_flux_rad<2><<<tile_grid(b, 64), 128, 0, c->stream>>>(G, b);
-      CKL("k_flux_rad<2>");
-    }
+    FLUX_DIR(0)
+    FLUX_DIR(1)
+    FLUX_DIR(2)
+#undef FLUX_DIR
+  }
+  if (!c->flux_split) {
+    // two blocks per SM loop over the queues
+    LaunchScope ls(c, K_FLUX_FIX);
+    k_flux_fix_all<<<2 * c->sm_count, 128, 0, c->stream>>>(G, F);
+    CKL("k_flux_fix_all");
   }
   Box eb{0, 0, 0, G.nx + 1, G.ny + 1, G.nz + 1};
   { LaunchScope ls(c, K_EMF); k_emf<<<nblocks(eb.n(), 128), 128, 0, c->stream>>>(G, eb); }
