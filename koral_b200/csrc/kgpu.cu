@@ -988,19 +988,6 @@ __device__ inline void count_lanes(unsigned long long *ctr, bool pred) {
   if (bits && (threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(ctr, (unsigned long long)__popc(bits));
 }
 
-// Floors, conserved from primitives and the stores that end a cell's
-// inversion (calc_primitives u2p.c:82-127).
-__device__ inline void u2p_finish(const Grid &G, long c, int ix, double *pp, double *uu, const Geom &g, int fix) {
-  Kin k;
-  bool kv;
-  check_floors_mhd(G, pp, g, G.rhofl_c ? G.rhofl_c[ix + G.ng] : -1., &k, &kv);
-  if (!kv) kinematics(pp, g, kMagn, k);
-  p2u_mhd(G, pp, uu, g, k);
-  store_cell(G.p, G.ncell, c, pp);
-  store_cell(G.u, G.ncell, c, uu);
-  G.flag[c] = fix;
-}
-
 // Warp-aggregated append to a work queue of box indices.
 __device__ inline void queue_push(int *queue, int *qcount, bool pred, int item) {
   const unsigned m = __activemask();
@@ -1019,13 +1006,53 @@ __device__ inline void count_sum(unsigned long long *ctr, unsigned v) {
   if (sum && (threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(ctr, (unsigned long long)sum);
 }
 
-// Queues of one inversion stage, reset by k_commit at the end of the stage.
+// Queues of one inversion stage, reset by the commit at the end of the stage.
 struct U2PQueues {
   int *slow, *ent, *slow_ent;      // box indices
-  int *n;                          // counts: [0] slow, [1] ent, [2] slow_ent
+  int *fix;                        // cells that asked for the neighbour fixup (G.flag set; clear everywhere else)
+  int *flo;                        // cells whose magnetic floor the first pass left to k_u2p_entropy
+  int *n;                          // counts: [0] slow, [1] ent, [2] slow_ent, [3] fix, [4] flo; [5] commit blocks done
   double *w;                       // saved W of a paused solve, per cell
   int *it;                         // saved iteration count, per cell
 };
+
+__device__ inline void request_fixup(const Grid &G, const U2PQueues &Q, long c, int item, bool pred) {
+  if (pred) G.flag[c] = 1;
+  queue_push(Q.fix, Q.n + 3, pred, item);
+}
+
+// Floors, conserved from primitives and the stores that end a cell's
+// inversion (calc_primitives u2p.c:82-127).  DEFER: a cell that needs the
+// magnetic floor (two nested W inversions, rare: the magnetised funnel) is
+// stored as it is and queued; k_u2p_entropy floors it with the same code.
+// The first pass, which every cell goes through, then has the registers of
+// its own inversion only (spilled bytes a thread at 5 blocks per SM: 872
+// stored and 2888 loaded before).
+template <bool DEFER>
+__device__ inline void u2p_finish(const Grid &G, const U2PQueues &Q, long c, int item, int ix, double *pp, double *uu,
+                                  const Geom &g) {
+  Kin k;
+  bool kv;
+  const double rfl = G.rhofl_c ? G.rhofl_c[ix + G.ng] : -1.;
+  if (DEFER) {
+    const double rho = pp[RHO], u = pp[UU];   // what the floors change before they reach the magnetic one
+    bool need = false;
+    check_floors_mhd(G, pp, g, rfl, &k, &kv, &need);
+    queue_push(Q.flo, Q.n + 4, need, item);
+    if (need) {
+      pp[RHO] = rho;
+      pp[UU] = u;
+      store_cell(G.p, G.ncell, c, pp);
+      return;
+    }
+  } else {
+    check_floors_mhd(G, pp, g, rfl, &k, &kv);
+  }
+  if (!kv) kinematics(pp, g, kMagn, k);
+  p2u_mhd(G, pp, uu, g, k);
+  store_cell(G.p, G.ncell, c, pp);
+  store_cell(G.u, G.ncell, c, uu);
+}
 
 // Cell state at the start of u2p (u2p.c:187-215): the conserved variables
 // (with the negative-density fix applied by the caller), the primitive
@@ -1060,7 +1087,8 @@ __device__ inline void u2p_load(const Grid &G, int ix, int iy, int iz, const dou
 // have taken, so per cell the arithmetic is that of u2p.  A cell whose
 // energy solve fails leaves its guess, as the solver left it, in pfix
 // (free until the fixup pass).
-__device__ inline void u2p_energy_done(const Grid &G, U2PQueues Q, int item, U2PCell &x, int r, int iter) {
+template <bool DEFER>
+__device__ inline void u2p_energy_done(const Grid &G, const U2PQueues &Q, int item, U2PCell &x, int r, int iter) {
   count_sum(&G.cnt[C_ITERS_HOT], (unsigned)iter);
   const bool failed = r < 0;
   queue_push(Q.ent, Q.n + 1, failed, item);
@@ -1071,11 +1099,12 @@ __device__ inline void u2p_energy_done(const Grid &G, U2PQueues Q, int item, U2P
   }
   const int fix = x.negrho ? 1 : 0;   // u2p's status stays -2 after a negative density
   count_lanes(&G.cnt[C_FIXUP], fix != 0);
+  request_fixup(G, Q, x.c, item, fix != 0);
   double uo[NVMAX];
-  u2p_finish(G, x.c, x.ix, x.pp, uo, x.g, fix);
+  u2p_finish<DEFER>(G, Q, x.c, item, x.ix, x.pp, uo, x.g);
 }
 
-__device__ inline void u2p_entropy_done(const Grid &G, U2PCell &x, int r, int iter) {
+__device__ inline void u2p_entropy_done(const Grid &G, const U2PQueues &Q, int item, U2PCell &x, int r, int iter) {
   count_sum(&G.cnt[C_ITERS_ENT], (unsigned)iter);
   int ret = -1;
   if (r < 0) {
@@ -1086,8 +1115,9 @@ __device__ inline void u2p_entropy_done(const Grid &G, U2PCell &x, int r, int it
   count_lanes(&G.cnt[C_FAIL], ret == -3);
   const int fix = ret < -1 ? 1 : 0;
   count_lanes(&G.cnt[C_FIXUP], fix != 0);
+  request_fixup(G, Q, x.c, item, fix != 0);
   double uo[NVMAX];
-  u2p_finish(G, x.c, x.ix, x.pp, uo, x.g, fix);
+  u2p_finish<false>(G, Q, x.c, item, x.ix, x.pp, uo, x.g);
 }
 
 // Damped-step halvings a first-pass solve may need before it is paused and
@@ -1118,7 +1148,6 @@ __global__ void __launch_bounds__(128, MB) k_u2p(Grid G, Box b, U2PQueues Q, int
     const long c = cell_index(G, ix, iy, iz);
     const double gdet = G.met_c[(long)(3 * 5 + 4) * G.nmet + met_index(G, ix, iy, iz)];
     for (int iv = B1; iv <= B3; iv++) G.p[iv * G.ncell + c] = G.u[iv * G.ncell + c] / gdet;
-    G.flag[c] = 0;
     return;
   }
   U2PCell x;
@@ -1139,7 +1168,7 @@ __global__ void __launch_bounds__(128, MB) k_u2p(Grid G, Box b, U2PQueues Q, int
     Q.it[x.c] = iter;
     return;
   }
-  u2p_energy_done(G, Q, t, x, r, iter);
+  u2p_energy_done<true>(G, Q, t, x, r, iter);
 }
 
 // Paused solves, one warp per cell (Etype 0: energy, 1: entropy).  All
@@ -1166,8 +1195,8 @@ __global__ void __launch_bounds__(128) k_u2p_resume(Grid G, Box b, U2PQueues Q, 
     int r = u2p_newton_warp(G.gamma, G.u2pconv, Etype, st.c, W, iter);
     if (r == 0) r = u2p_final(G.gamma, st, W, iter, x.uc, x.pp, x.g);
     if (lane == 0) {
-      if (Etype == 0) u2p_energy_done(G, Q, item, x, r, iter);
-      else u2p_entropy_done(G, x, r, iter);
+      if (Etype == 0) u2p_energy_done<false>(G, Q, item, x, r, iter);
+      else u2p_entropy_done(G, Q, item, x, r, iter);
     }
     __syncwarp();
   }
@@ -1192,7 +1221,20 @@ __global__ void __launch_bounds__(128) k_u2p_entropy(Grid G, Box b, U2PQueues Q,
       Q.it[x.c] = iter;
       continue;
     }
-    u2p_entropy_done(G, x, r, iter);
+    u2p_entropy_done(G, Q, item, x, r, iter);
+  }
+  // the magnetic floors that the first pass left
+  const int nf = Q.n[4];
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nf; q += gridDim.x * blockDim.x) {
+    int ix, iy, iz;
+    const int item = Q.flo[q];
+    box_coord(b, item, ix, iy, iz);
+    const long c = cell_index(G, ix, iy, iz);
+    double pp[NVMAX], uu[NVMAX];
+    Geom g;
+    load_cell(G.p, G.ncell, c, pp);
+    geom_centre(G, ix, iy, iz, g);
+    u2p_finish<false>(G, Q, c, item, ix, pp, uu, g);
   }
 }
 
@@ -1267,19 +1309,16 @@ __global__ void k_imp_gather(Grid G, Box b, const double *dtp, double fac, doubl
   }
   dt[k] = (dtp[0] * fac) * 1.;
 }
-__global__ void k_imp_scatter(Grid G, Box b, const double *pp, const double *uu, const int *status) {
+__global__ void k_imp_scatter(Grid G, Box b, U2PQueues Q, const double *pp, const double *uu, const int *status) {
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
   int ix, iy, iz;
   if (!box_coord(b, k, ix, iy, iz)) return;
   const long c = cell_index(G, ix, iy, iz);
-  if (polar_cell(G, iy)) {   // op_implicit skips corrected polar cells (finite.c:1270-1272)
-    G.flag[c] = 0;
-    return;
-  }
+  if (polar_cell(G, iy)) return;   // op_implicit skips corrected polar cells (finite.c:1270-1272)
   const bool ok = status[k] == 0;
   count_lanes(&G.cnt[C_RADIMP_FAIL], !ok);
   count_lanes(&G.cnt[C_IMP_SOLVES], true);
-  G.flag[c] = ok ? 0 : 1;
+  request_fixup(G, Q, c, (int)k, !ok);
   if (!ok) return;
 #pragma unroll
   for (int iv = 0; iv < NVR; iv++) {
@@ -1343,11 +1382,10 @@ __global__ void k_imex_final(Grid G, Box b, const double *dtp, const double *ut0
 // each flag as it goes, so a neighbour that precedes the cell in that order
 // always counts as good, one that follows counts when its own inversion
 // succeeded.  Neighbour values are the post-inversion primitives.
-__global__ void k_fixup(Grid G, Box b, int *fixmark) {
-  int ix, iy, iz;
-  if (!box_coord(b, blockIdx.x * (long)blockDim.x + threadIdx.x, ix, iy, iz)) return;
+// Only the cells that asked for it are visited (a queue of a few to a few
+// thousand cells).
+__device__ inline void fixup_cell(const Grid &G, int ix, int iy, int iz, int *fixmark) {
   const long c = cell_index(G, ix, iy, iz);
-  if (G.flag[c] == 0) return;
   const int NX = G.nx, NY = G.ny, NZ = G.nz;
   constexpr int nv = NVMAX;
   int nb[6][3] = {{ix - 1, iy, iz}, {ix + 1, iy, iz}, {ix, iy - 1, iz}, {ix, iy + 1, iz}, {ix, iy, iz - 1}, {ix, iy, iz + 1}};
@@ -1378,30 +1416,50 @@ __global__ void k_fixup(Grid G, Box b, int *fixmark) {
   store_cell(G.ufix, G.ncell, c, uu);
   fixmark[c] = 1;
 }
+__global__ void k_fixup(Grid G, Box b, U2PQueues Q, int *fixmark) {
+  const int n = Q.n[3];
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    int ix, iy, iz;
+    box_coord(b, Q.fix[q], ix, iy, iz);
+    fixup_cell(G, ix, iy, iz, fixmark);
+  }
+}
 
-// apply fixups; optionally finish an RK2 step: u = ut0 + (u - ut1)
-// (addi_u pair of ko.c:614-615)
-__global__ void k_commit(Grid G, Box b, const int *fixmark, int combine, int *qcount) {
-  if (blockIdx.x == 0 && threadIdx.x < 3) qcount[threadIdx.x] = 0;   // the inversion queues of this stage are spent
-  int ix, iy, iz;
-  if (!box_coord(b, blockIdx.x * (long)blockDim.x + threadIdx.x, ix, iy, iz)) return;
-  const long c = cell_index(G, ix, iy, iz);
-  constexpr int nv = NVMAX;
-  if (G.flag[c] != 0) {
-    if (fixmark[c]) {
-      for (int iv = 0; iv < nv; iv++) {
+// Applies the fixups of the queued cells and empties the queues of the stage.
+// The last block to finish empties the fixup queue itself.
+__global__ void k_commit(Grid G, Box b, U2PQueues Q, const int *fixmark) {
+  if (blockIdx.x == 0 && (threadIdx.x < 3 || threadIdx.x == 4)) Q.n[threadIdx.x] = 0;
+  const int n = *(volatile int *)(Q.n + 3);
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    int ix, iy, iz;
+    box_coord(b, Q.fix[q], ix, iy, iz);
+    const long c = cell_index(G, ix, iy, iz);
+    if (fixmark[c])
+      for (int iv = 0; iv < NVMAX; iv++) {
         G.p[iv * G.ncell + c] = G.pfix[iv * G.ncell + c];
         G.u[iv * G.ncell + c] = G.ufix[iv * G.ncell + c];
       }
-    }
     G.flag[c] = 0;
   }
-  if (combine) {
-    for (int iv = 0; iv < nv; iv++) {
-      long i = iv * G.ncell + c;
-      double ut2 = 1. * G.u[i] + (-1.) * G.ut1[i];
-      G.u[i] = 1. * G.ut0[i] + 1. * ut2;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(Q.n + 5, 1) == (int)gridDim.x - 1) {   // every block has read the count
+      Q.n[3] = 0;
+      Q.n[5] = 0;
     }
+  }
+}
+// The end of an RK2 step: u = ut0 + (u - ut1) (addi_u pair of ko.c:614-615)
+__global__ void k_combine(Grid G, Box b) {
+  int ix, iy, iz, item;
+  if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) return;
+  const long c = cell_index(G, ix, iy, iz);
+#pragma unroll
+  for (int iv = 0; iv < NVMAX; iv++) {
+    const long i = iv * G.ncell + c;
+    const double ut2 = 1. * G.u[i] + (-1.) * G.ut1[i];
+    G.u[i] = 1. * G.ut0[i] + 1. * ut2;
   }
 }
 
@@ -1913,7 +1971,9 @@ extern "C" int kgpu_create(const kgpu_config *cfg, kgpu_ctx **out) {
   AL(c->u2pq.slow, G.ncell * sizeof(int));
   AL(c->u2pq.ent, G.ncell * sizeof(int));
   AL(c->u2pq.slow_ent, G.ncell * sizeof(int));
-  AL(c->u2pq.n, 4 * sizeof(int));
+  AL(c->u2pq.fix, G.ncell * sizeof(int));
+  AL(c->u2pq.flo, G.ncell * sizeof(int));
+  AL(c->u2pq.n, 8 * sizeof(int));
   AL(c->u2pq.w, G.ncell * d8);
   AL(c->u2pq.it, G.ncell * sizeof(int));
   AL(G.scal, S_NSCAL * d8);
@@ -1938,7 +1998,7 @@ extern "C" int kgpu_create(const kgpu_config *cfg, kgpu_ctx **out) {
   CK(cudaMemsetAsync(G.emf, 0, 3L * (G.nx + 1) * (G.ny + 1) * (G.nz + 1) * d8, c->stream));
   CK(cudaMemsetAsync(G.flag, 0, G.ncell * sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->fixmark, 0, G.ncell * sizeof(int), c->stream));
-  CK(cudaMemsetAsync(c->u2pq.n, 0, 4 * sizeof(int), c->stream));
+  CK(cudaMemsetAsync(c->u2pq.n, 0, 8 * sizeof(int), c->stream));
   CK(cudaMemsetAsync(G.scal, 0, S_NSCAL * d8, c->stream));
   CK(cudaMemsetAsync(G.cnt, 0, C_NCNT * sizeof(unsigned long long), c->stream));
   CK(cudaMemsetAsync((void *)G.gkr, 0, G.nmet * 64 * d8, c->stream));
@@ -2375,10 +2435,14 @@ static int launch_u2p(kgpu_ctx *c, int combine) {
     { LaunchScope ls(c, K_U2P_RAD); k_u2p_rad<<<tile_grid(db, 128), 128, 0, c->stream>>>(G, db); }
     CKL("k_u2p_rad");
   }
-  { LaunchScope ls(c, K_FIXUP); k_fixup<<<nblocks(db.n(), 128), 128, 0, c->stream>>>(G, db, c->fixmark); }
+  { LaunchScope ls(c, K_FIXUP); k_fixup<<<c->sm_count, 128, 0, c->stream>>>(G, db, c->u2pq, c->fixmark); }
   CKL("k_fixup");
-  { LaunchScope ls(c, K_COMMIT); k_commit<<<nblocks(db.n(), 256), 256, 0, c->stream>>>(G, db, c->fixmark, combine, c->u2pq.n); }
+  { LaunchScope ls(c, K_COMMIT); k_commit<<<c->sm_count, 128, 0, c->stream>>>(G, db, c->u2pq, c->fixmark); }
   CKL("k_commit");
+  if (combine) {
+    { LaunchScope ls(c, K_COMMIT); k_combine<<<tile_grid(db, 128), 128, 0, c->stream>>>(G, db); }
+    CKL("k_combine");
+  }
   return launch_bc(c);
 }
 
@@ -2768,11 +2832,11 @@ static int enqueue_implicit(kgpu_ctx *c, const double *dtp, double fac) {
     c->launches += nl - 1;
   }
   { LaunchScope ls(c, K_IMP_SCATTER);
-    k_imp_scatter<<<nblocks(db.n(), 128), 128, 0, c->stream>>>(G, db, c->imp_ppo, c->imp_uuo, c->imp_status); }
+    k_imp_scatter<<<nblocks(db.n(), 128), 128, 0, c->stream>>>(G, db, c->u2pq, c->imp_ppo, c->imp_uuo, c->imp_status); }
   CKL("k_imp_scatter");
-  { LaunchScope ls(c, K_FIXUP); k_fixup<<<nblocks(db.n(), 128), 128, 0, c->stream>>>(G, db, c->fixmark); }
+  { LaunchScope ls(c, K_FIXUP); k_fixup<<<c->sm_count, 128, 0, c->stream>>>(G, db, c->u2pq, c->fixmark); }
   CKL("k_fixup");
-  { LaunchScope ls(c, K_COMMIT); k_commit<<<nblocks(db.n(), 256), 256, 0, c->stream>>>(G, db, c->fixmark, 0, c->u2pq.n); }
+  { LaunchScope ls(c, K_COMMIT); k_commit<<<c->sm_count, 128, 0, c->stream>>>(G, db, c->u2pq, c->fixmark); }
   CKL("k_commit");
   return 0;
 }
@@ -3013,13 +3077,8 @@ extern "C" int kgpu_autotune(kgpu_ctx *c, int steps, double min_gain, int reuse,
     std::vector<Knob> round = {knobs[ki]};
     // the settings that belong to the solver form just chosen
     if (G.rad && knobs[ki].field(best) == &best.implicit.inner_cap) {
-      if (best.implicit_mode == KGPU_RAD_BATCHED) {
-        round.push_back({[](kgpu_tuning &t) { return &t.implicit.pass_iters; }, {4, 8, 16}});
-        round.push_back({[](kgpu_tuning &t) { return &t.implicit.tail; }, {0, 4, 8, 16}});
-        round.push_back({[](kgpu_tuning &t) { return &t.implicit.hard; }, {-1, 8, 16, 32}});
-      } else {
+      if (best.implicit_mode == KGPU_RAD_PERSISTENT)
         round.push_back({[](kgpu_tuning &t) { return &t.implicit.thin; }, {4, 8, 16}});
-      }
     }
     for (const Knob &kn : round) {
       std::vector<double> ms;
