@@ -636,7 +636,7 @@ KG_HD int u2p_bracket(double GAMMA, int Etype, const U2PCons &c, double &W, U2PF
 // evaluation is passed on to the next iteration by shuffles instead of being
 // done again, which halves the chain of dependent evaluations.
 __device__ inline int u2p_newton_warp(double GAMMA, double CONV, int Etype, const U2PCons &c, double &W, int &iter,
-                                      U2PF F = U2PF{0., 0., 0.}, bool have = false) {
+                                      U2PF F = U2PF{0., 0., 0.}, bool have = false, unsigned *fevals = nullptr) {
   const int lane = threadIdx.x & 31;
   const double D = c.D;
   U2PF S{0., 0., 0.};      // the function where the running step started
@@ -644,6 +644,7 @@ __device__ inline int u2p_newton_warp(double GAMMA, double CONV, int Etype, cons
   if (have) {
     S = F;
     iter++;
+    if (fevals) (*fevals)++;
     if (S.err < CONV) return 0;
     base = 0;
   }
@@ -665,6 +666,7 @@ __device__ inline int u2p_newton_warp(double GAMMA, double CONV, int Etype, cons
     if (base < 0) {
       S = T;
       iter++;
+      if (fevals) (*fevals)++;
       if (S.err < CONV) return 0;
       base = 0;
       continue;
@@ -677,6 +679,7 @@ __device__ inline int u2p_newton_warp(double GAMMA, double CONV, int Etype, cons
       continue;
     }
     const int L = __ffs(m) - 1;
+    if (fevals) *fevals += (unsigned)(base + L + 1);   // the trials of the scalar loop
     if (base + L >= 100) return -101;
     const double Wprev = W, err = S.err;
     W = __shfl_sync(0xffffffffu, at, L);
@@ -687,6 +690,7 @@ __device__ inline int u2p_newton_warp(double GAMMA, double CONV, int Etype, cons
     if (fabs((W - Wprev) / Wprev) < CONV && err < 1.e-1) return 0;
     if (!(iter < 50)) return 0;
     iter++;
+    if (fevals) (*fevals)++;
     if (S.err < CONV) return 0;
     base = 0;
   }

@@ -103,6 +103,204 @@ __device__ int u2p_counted(const Grid &G, const double *uu0, double *pp, const G
   return ret;
 }
 
+// ---------------------------------------------------------------------------
+// The inversion without a prediction, in two launches.  One thread per cell
+// through both equations made every warp as slow as its slowest cell: on
+// 1048576 magnetised cells, 1% of which end in the entropy equation, 4.9 of
+// 32 lanes were active on average and a launch took 3.8 ms.  Now k_u2p_first
+// gives every cell the energy equation with the limits of the grid's first
+// pass and marks the cells that need more in their status; k_u2p_rest gathers
+// those, block by block over a range of cells, and gives the paused solves a
+// warp each and the entropy solves a thread each, with the same limits, and
+// then a warp each.  Per cell the same steps are taken, so results and
+// counters are the same.  No memory besides the outputs is needed.
+// ---------------------------------------------------------------------------
+enum : int { CELL_PAUSED = 1001, CELL_ENTROPY = 1002, CELL_WHOLE = 1003 };   // no status u2p returns
+constexpr int FIRST_STEPS = 8, FIRST_HALVINGS = 4;
+
+__device__ inline void add_stats(unsigned long long *stats, unsigned it, unsigned fell, unsigned fe) {
+  const unsigned m = __activemask();
+  const unsigned a = __reduce_add_sync(m, it), b = __reduce_add_sync(m, fell), c = __reduce_add_sync(m, fe);
+  if ((threadIdx.x & 31) == __ffs(m) - 1) {
+    if (a) atomicAdd(&stats[0], (unsigned long long)a);
+    if (b) atomicAdd(&stats[1], (unsigned long long)b);
+    if (c) atomicAdd(&stats[2], (unsigned long long)c);
+  }
+}
+
+// the cell as u2p starts on it; true where its density was negative
+__device__ inline bool cell_load(const Grid &G, int nv, const double *uu, const double *pp, long i, const Geom &g,
+                                 double *u, double *p) {
+  for (int iv = 0; iv < NVMAX; iv++) {
+    u[iv] = uu[i * nv + iv];
+    p[iv] = pp[i * nv + iv];
+  }
+  if (!(u[0] / g.gdet < 0.)) return false;
+  p[0] = G.rhofloor;
+  u[0] = G.rhofloor * g.gdet;
+  return true;
+}
+__device__ inline void cell_store(int nv, double *pp, long i, const double *p, int ret, int it, int *status,
+                                  int *fixup, int *iters) {
+  if (ret != -3)
+    for (int iv = 0; iv < NVMAX; iv++) pp[i * nv + iv] = p[iv];   // a failure keeps the guess
+  status[i] = ret;
+  fixup[i] = ret < -1 ? 1 : 0;
+  if (iters) iters[i] = it;
+}
+
+__global__ void __launch_bounds__(128, 4) k_u2p_first(U2PParams P, int n, int nv, const double *uu, double *pp,
+                                                      const double *g20, const double *G20, int *status, int *fixup,
+                                                      int *iters, unsigned long long *stats) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const Grid G = u2p_grid(P);
+  Geom g;
+  cell_geom(g20, G20, i, g);
+  double u[NVMAX], p[NVMAX];
+  const bool negrho = cell_load(G, nv, uu, pp, i, g, u, p);
+  U2PState s;
+  u2p_setup(u, g, s);
+  double W = u2p_initial_w(G.gamma, p, g);
+  int it = 0;
+  unsigned fe = 0;
+  int r = u2p_solve_w(G.gamma, G.u2pconv, 0, s.c, W, it, FIRST_STEPS, FIRST_HALVINGS, &fe);
+  const bool paused = r == U2P_PAUSED;
+  if (r == 0) r = u2p_final(G.gamma, s, W, it, u, p, g);
+  if (paused) {
+    status[i] = CELL_PAUSED;   // its solve is done again from the start
+  } else if (r < 0) {
+    // what a failed solve leaves in the primitives is read by the next: only
+    // the check on the density fails after they are set
+    status[i] = r == -105 ? CELL_WHOLE : CELL_ENTROPY;
+    fixup[i] = it;
+  } else {
+    cell_store(nv, pp, i, p, negrho ? -2 : 0, it, status, fixup, iters);
+  }
+  const bool count = !paused && r != -105;
+  if (stats) add_stats(stats, count ? it : 0, 0, count ? fe : 0);
+}
+
+// a warp on the whole solve of equation Etype of one cell; every lane returns
+// the same values
+__device__ inline int solve_warp(const Grid &G, const double *u, double *p, const Geom &g, int Etype, int &it,
+                                 unsigned &fe) {
+  U2PState s;
+  u2p_setup(u, g, s);
+  double W = u2p_initial_w(G.gamma, p, g);
+  U2PF F;
+  if (u2p_bracket(G.gamma, Etype, s.c, W, F, &fe)) return -150;
+  int k = 0;
+  const int r = u2p_newton_warp(G.gamma, G.u2pconv, Etype, s.c, W, k, F, true, &fe);
+  it += k;
+  if (r < 0) return r;
+  return u2p_final(G.gamma, s, W, k, u, p, g);
+}
+
+constexpr int REST_THREADS = 128, REST_RANGE = 4096;
+
+__global__ void __launch_bounds__(REST_THREADS) k_u2p_rest(U2PParams P, int n, int nv, int range, const double *uu,
+                                                           double *pp, const double *g20, const double *G20,
+                                                           int *status, int *fixup, int *iters,
+                                                           unsigned long long *stats) {
+  __shared__ int cell[REST_RANGE];   // paused from the front, to the entropy equation from the back
+  __shared__ int na, nb;
+  const Grid G = u2p_grid(P);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i0 = blockIdx.x * range, i1 = i0 + range < n ? i0 + range : n;
+  if (tid == 0) na = nb = 0;
+  __syncthreads();
+  for (int i = i0 + tid; i < i1; i += REST_THREADS) {
+    const int st = status[i];
+    if (st == CELL_PAUSED) cell[atomicAdd(&na, 1)] = i;
+    else if (st == CELL_ENTROPY || st == CELL_WHOLE) cell[range - 1 - atomicAdd(&nb, 1)] = i;
+  }
+  __syncthreads();
+  // paused energy solves, a warp each; one that fails is marked for the
+  // entropy equation
+  const int n1 = na, n2 = nb;
+  for (int q = warp; q < n1; q += REST_THREADS / 32) {
+    const int i = cell[q];
+    Geom g;
+    cell_geom(g20, G20, i, g);
+    double u[NVMAX], p[NVMAX];
+    const bool negrho = cell_load(G, nv, uu, pp, i, g, u, p);
+    int it = 0;
+    unsigned fe = 0;
+    const int r = solve_warp(G, u, p, g, 0, it, fe);
+    __syncwarp();
+    if (lane == 0) {
+      if (r < 0) {
+        status[i] = r == -105 ? CELL_WHOLE : CELL_ENTROPY;
+        fixup[i] = it;
+      } else {
+        cell_store(nv, pp, i, p, negrho ? -2 : 0, it, status, fixup, iters);
+      }
+      if (stats && !(r == -105)) add_stats(stats, it, 0, fe);
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+  // entropy solves, a thread each, over both lists; the paused ones are
+  // marked and stay for the warps
+  const int total = n1 + n2;
+  for (int q = tid; q < total; q += REST_THREADS) {
+    const int i = cell[q < n2 ? range - 1 - q : q - n2];
+    const int st = status[i];
+    if (st == CELL_WHOLE || st == CELL_ENTROPY) {
+      Geom g;
+      cell_geom(g20, G20, i, g);
+      double u[NVMAX], p[NVMAX];
+      if (st == CELL_WHOLE) {
+        for (int iv = 0; iv < NVMAX; iv++) {
+          u[iv] = uu[(long)i * nv + iv];
+          p[iv] = pp[(long)i * nv + iv];
+        }
+        int fix = 0;
+        unsigned it = 0, fe = 0;
+        const int ret = u2p_counted(G, u, p, g, fix, -1., false, it, fe);
+        cell_store(nv, pp, i, p, ret, (int)it, status, fixup, iters);
+        if (stats) add_stats(stats, it, 0, fe);
+      } else {
+        cell_load(G, nv, uu, pp, i, g, u, p);
+        U2PState s;
+        u2p_setup(u, g, s);
+        double W = u2p_initial_w(G.gamma, p, g);
+        int it = 0;
+        unsigned fe = 0;
+        int r = u2p_solve_w(G.gamma, G.u2pconv, 1, s.c, W, it, FIRST_STEPS, FIRST_HALVINGS, &fe);
+        const bool paused = r == U2P_PAUSED;
+        if (r == 0) r = u2p_final(G.gamma, s, W, it, u, p, g);
+        if (paused) {
+          status[i] = CELL_PAUSED;
+        } else {
+          cell_store(nv, pp, i, p, r < 0 ? -3 : -1, fixup[i] + it, status, fixup, iters);
+          if (stats) add_stats(stats, it, 0, fe);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int q = warp; q < total; q += REST_THREADS / 32) {
+    const int i = cell[q < n2 ? range - 1 - q : q - n2];
+    if (status[i] != CELL_PAUSED) continue;
+    Geom g;
+    cell_geom(g20, G20, i, g);
+    double u[NVMAX], p[NVMAX];
+    cell_load(G, nv, uu, pp, i, g, u, p);
+    int it = 0;
+    unsigned fe = 0;
+    const int r = solve_warp(G, u, p, g, 1, it, fe);
+    __syncwarp();   // every lane has read the status
+    if (lane == 0) {
+      cell_store(nv, pp, i, p, r < 0 ? -3 : -1, fixup[i] + it, status, fixup, iters);
+      if (stats) add_stats(stats, it, 0, fe);
+    }
+    __syncwarp();
+  }
+}
+
+// The inversion from a prediction, one thread per cell
 __global__ void k_u2p_warm_cells(U2PParams P, int n, int nv, const double *uu, double *pp, const double *g20,
                                  const double *G20, const float *ypred, float wgate, float sgate, int *status,
                                  int *fixup, int *iters, unsigned long long *stats) {
@@ -118,9 +316,7 @@ __global__ void k_u2p_warm_cells(U2PParams P, int n, int nv, const double *uu, d
       p[iv] = p0[iv] = pp[(long)i * nv + iv];
     }
     int fix = 0, ret;
-    if (!ypred) {
-      ret = u2p_counted(G, u, p, g, fix, -1., false, it, fe);
-    } else {
+    {
       const float *y = ypred + (long)i * MLP_OUTP;
       // a predicted change of W smaller than wgate is within the network's
       // own error: the guess's W is kept; the energy equation is skipped
@@ -226,9 +422,24 @@ extern "C" int kgpu_u2p_cells_device(int n, const kgpu_config *cfg, int nv, cons
     WCK(cudaMallocAsync(&dstats, 3 * sizeof(unsigned long long), s));
     WCK(cudaMemsetAsync(dstats, 0, 3 * sizeof(unsigned long long), s));
   }
-  k_u2p_warm_cells<<<(n + 127) / 128, 128, 0, s>>>(P, n, nv, uu, pp, g, G, ypred, wgate, sgate, status, fixup, iters,
-                                                    dstats);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e;
+  if (ypred) {
+    k_u2p_warm_cells<<<(n + 127) / 128, 128, 0, s>>>(P, n, nv, uu, pp, g, G, ypred, wgate, sgate, status, fixup, iters,
+                                                      dstats);
+    e = cudaGetLastError();
+  } else {
+    k_u2p_first<<<(n + 127) / 128, 128, 0, s>>>(P, n, nv, uu, pp, g, G, status, fixup, iters, dstats);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) {
+      // a range per block: as many blocks as two per SM hold, so that a
+      // block's few hard cells fill more of its lanes, down to a range of 128
+      int range = (n + 2 * 148 - 1) / (2 * 148);
+      range = range < REST_THREADS ? REST_THREADS : (range > REST_RANGE ? REST_RANGE : range);
+      k_u2p_rest<<<(n + range - 1) / range, REST_THREADS, 0, s>>>(P, n, nv, range, uu, pp, g, G, status, fixup, iters,
+                                                                   dstats);
+      e = cudaGetLastError();
+    }
+  }
   if (dstats) {
     unsigned long long h[3] = {0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, dstats, sizeof(h), cudaMemcpyDeviceToHost, s);
