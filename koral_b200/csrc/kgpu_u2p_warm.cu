@@ -22,6 +22,8 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include <map>
+
 #include "../../include/koral_b200.h"
 #include "kgpu_mlp.cuh"
 
@@ -197,7 +199,9 @@ __device__ inline int solve_warp(const Grid &G, const double *u, double *p, cons
   return u2p_final(G.gamma, s, W, k, u, p, g);
 }
 
-constexpr int REST_THREADS = 128, REST_RANGE = 4096;
+// cells a block of the second launch looks over: 1.47 ms for 2^20 cells at
+// 1024, 1.55 at 512 (fewer hard cells to a warp), 1.60 at 2048 (fewer blocks)
+constexpr int REST_THREADS = 128, REST_RANGE = 1024;
 
 __global__ void __launch_bounds__(REST_THREADS) k_u2p_rest(U2PParams P, int n, int nv, int range, const double *uu,
                                                            double *pp, const double *g20, const double *G20,
@@ -383,6 +387,27 @@ bool params_of(const kgpu_config *cfg, int nv, U2PParams &P) {
   return true;
 }
 
+// The counters of a call that reports them: one small buffer per host thread
+// and device, free again when the call has synchronised, given back when the
+// thread ends.  (A stream-ordered allocation went back to the driver at every
+// synchronisation, and mapping it anew cost a few hundred microseconds.)
+struct ThreadCounters {
+  std::map<int, unsigned long long *> of_device;
+  ~ThreadCounters() {
+    for (auto &kv : of_device) cudaFree(kv.second);
+  }
+};
+cudaError_t thread_counters(unsigned long long **p) {
+  static thread_local ThreadCounters mine;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  unsigned long long *&q = mine.of_device[dev];
+  if (!q && (e = cudaMalloc(&q, 3 * sizeof(unsigned long long))) != cudaSuccess) return e;
+  *p = q;
+  return cudaSuccess;
+}
+
 }  // namespace
 
 extern "C" int kgpu_u2p_features_device(int n, const kgpu_config *cfg, int nv, const double *uu, const double *pp,
@@ -419,7 +444,7 @@ extern "C" int kgpu_u2p_cells_device(int n, const kgpu_config *cfg, int nv, cons
   cudaStream_t s = (cudaStream_t)stream;
   unsigned long long *dstats = nullptr;
   if (nstats > 0) {
-    WCK(cudaMallocAsync(&dstats, 3 * sizeof(unsigned long long), s));
+    WCK(thread_counters(&dstats));
     WCK(cudaMemsetAsync(dstats, 0, 3 * sizeof(unsigned long long), s));
   }
   cudaError_t e;
@@ -443,7 +468,6 @@ extern "C" int kgpu_u2p_cells_device(int n, const kgpu_config *cfg, int nv, cons
   if (dstats) {
     unsigned long long h[3] = {0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, dstats, sizeof(h), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(dstats, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     for (int k = 0; k < nstats; k++) stats[k] = h[k];
   }
