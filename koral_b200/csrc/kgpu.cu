@@ -111,6 +111,32 @@ __device__ inline bool tile_coord(const Box &b, int per_block, int e, int &ix, i
   item = (int)(pl + (unsigned)z * (unsigned)(b.nx * b.ny));
   return true;
 }
+// The kernels of a step are launched on the stream with programmatic
+// serialisation: the next one is brought up (its blocks placed, its parameters
+// read) while the one before still runs, and waits here, before it touches
+// memory, until that one has completed.  Every thread of every such kernel
+// begins with this call, so a kernel completes only after the one before it
+// has.  Four steps of the 16x16 vortex driven operator by operator: 1295 ->
+// 1057 us.  Inside a captured step it gained nothing (40 steps of the 128x128
+// vortex 6.00 against 6.13 ms), so a capture launches as usual.
+static thread_local bool g_capturing = false;
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+static void launch_next(cudaStream_t st, dim3 grid, int block, void (*kernel)(P...), A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = g_capturing ? 0 : 1;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);   // an error stays for the caller's cudaGetLastError
+}
 static inline unsigned nblocks(long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 __device__ inline bool in_domain(const Grid &G, int ix, int iy, int iz) {
@@ -264,6 +290,7 @@ static BcParts bc_parts(const Grid &G) {
 }
 
 __global__ void __launch_bounds__(128) k_bc(Grid G, BcParts P) {
+  after_previous();
   int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   int part = 0;
   while (part < 7 && t >= P.n[part]) t -= P.n[part++];
@@ -367,6 +394,7 @@ __device__ inline void atomic_max_pos(double *addr, double v) {
 }
 
 __global__ void k_wavespeeds(Grid G, Box b) {
+  after_previous();
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 3) G.fqn[threadIdx.x] = 0;   // the flux kernels' queues
   int ix, iy, iz, item;
   double tsd = -1.;
@@ -460,6 +488,7 @@ __global__ void k_wavespeeds(Grid G, Box b) {
 // same functions and operations as the reconstruction inside k_flux.
 template <int D>
 __global__ void __launch_bounds__(256) k_recon(Grid G, Box b, double *sl, double *sr) {
+  after_previous();
   const long nb = b.n();
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (t >= nb * NVMAX) return;
@@ -602,6 +631,7 @@ __device__ __forceinline__ void face_flux(const Grid &G, const Box &b, const dou
 
 template <int D, int MB = KGPU_FLUX_MIN_BLOCKS, bool SPLIT = false>
 __global__ void __launch_bounds__(128, MB) k_flux(Grid G, Box b, const double *sl, const double *sr) {
+  after_previous();
   int ix, iy, iz, fi;
   const bool valid = tile_coord(b, 64, threadIdx.x >> 1, ix, iy, iz, fi);
   const unsigned pairmask = __ballot_sync(0xffffffffu, valid);
@@ -618,6 +648,7 @@ struct FaceBoxes {
   unsigned gx[3], n[3];   // tiles of the plane; blocks
 };
 __global__ void __launch_bounds__(128, 4) k_flux_all(Grid G, FaceBoxes F) {
+  after_previous();
   const unsigned t0 = blockIdx.x;
   const int d = t0 < F.n[0] ? 0 : (t0 < F.n[0] + F.n[1] ? 1 : 2);
   const unsigned t = t0 - (d > 0 ? F.n[0] : 0u) - (d > 1 ? F.n[1] : 0u);
@@ -656,10 +687,12 @@ __device__ __forceinline__ void flux_fix(const Grid &G, const Box &b, const doub
 // one direction (the split form reuses its face states for the next one)
 template <int D>
 __global__ void __launch_bounds__(128) k_flux_fix(Grid G, Box b, const double *sl, const double *sr) {
+  after_previous();
   flux_fix<D, true>(G, b, sl, sr);
 }
 // all directions, their queues one after another: empty on most steps
 __global__ void __launch_bounds__(128) k_flux_fix_all(Grid G, FaceBoxes F) {
+  after_previous();
   if (F.n[0]) flux_fix<0, false>(G, F.b[0], nullptr, nullptr);
   if (F.n[1]) flux_fix<1, false>(G, F.b[1], nullptr, nullptr);
   if (F.n[2]) flux_fix<2, false>(G, F.b[2], nullptr, nullptr);
@@ -736,6 +769,7 @@ __device__ __forceinline__ void face_flux_rad(const Grid &G, int ix, int iy, int
 
 template <int D>
 __global__ void __launch_bounds__(128) k_flux_rad(Grid G, Box b) {
+  after_previous();
   int ix, iy, iz, fi;
   const bool valid = tile_coord(b, 64, threadIdx.x >> 1, ix, iy, iz, fi);
   const unsigned pairmask = __ballot_sync(0xffffffffu, valid);
@@ -743,6 +777,7 @@ __global__ void __launch_bounds__(128) k_flux_rad(Grid G, Box b) {
 }
 // the three directions in one launch, as k_flux_all
 __global__ void __launch_bounds__(128) k_flux_rad_all(Grid G, FaceBoxes F) {
+  after_previous();
   const unsigned t0 = blockIdx.x;
   const int d = t0 < F.n[0] ? 0 : (t0 < F.n[0] + F.n[1] ? 1 : 2);
   const unsigned t = t0 - (d > 0 ? F.n[0] : 0u) - (d > 1 ? F.n[1] : 0u);
@@ -780,6 +815,7 @@ struct Acc {
 };
 
 __global__ void k_emf(Grid G, Box b) {
+  after_previous();
   int ix, iy, iz;
   if (!box_coord(b, blockIdx.x * (long)blockDim.x + threadIdx.x, ix, iy, iz)) return;
   const int NX = G.nx, NY = G.ny, NZ = G.nz;
@@ -823,6 +859,7 @@ __global__ void k_emf(Grid G, Box b) {
 template <int MB = KGPU_UPDATE_MIN_BLOCKS>
 __global__ void __launch_bounds__(128, MB) k_update(Grid G, Box b, const double *dtp, double fac,
                                                                         double *save) {
+  after_previous();
   int ix, iy, iz, item;
   if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) return;
   constexpr int nv = NVMAX;
@@ -934,6 +971,7 @@ __global__ void __launch_bounds__(128, MB) k_update(Grid G, Box b, const double 
 // over EE0..FZ0): flux divergence plus the radiative metric source
 // gdet R^k_l Gamma^l_{jk} (f_metric_source_term_arb, physics.c:383-405).
 __global__ void __launch_bounds__(128) k_update_rad(Grid G, Box b, const double *dtp, double fac) {
+  after_previous();
   int ix, iy, iz, item;
   if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) return;
   const long c = cell_index(G, ix, iy, iz);
@@ -1139,6 +1177,7 @@ __device__ inline int u2p_run(const Grid &G, int Etype, U2PCell &x, int stop, do
 
 template <int MB = KGPU_U2P_MIN_BLOCKS>
 __global__ void __launch_bounds__(128, MB) k_u2p(Grid G, Box b, U2PQueues Q, int stop) {
+  after_previous();
   int ix, iy, iz, t;
   if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, t)) return;
   if (polar_cell(G, iy)) {
@@ -1174,6 +1213,7 @@ __global__ void __launch_bounds__(128, MB) k_u2p(Grid G, Box b, U2PQueues Q, int
 // Paused solves, one warp per cell (Etype 0: energy, 1: entropy).  All
 // lanes carry the cell; lane 0 writes the outcome.
 __global__ void __launch_bounds__(128) k_u2p_resume(Grid G, Box b, U2PQueues Q, int Etype) {
+  after_previous();
   const int n = Q.n[Etype == 0 ? 0 : 2];
   const int *queue = Etype == 0 ? Q.slow : Q.slow_ent;
   const int lane = threadIdx.x & 31;
@@ -1203,6 +1243,7 @@ __global__ void __launch_bounds__(128) k_u2p_resume(Grid G, Box b, U2PQueues Q, 
 }
 
 __global__ void __launch_bounds__(128) k_u2p_entropy(Grid G, Box b, U2PQueues Q, int stop) {
+  after_previous();
   const int n = Q.n[1];
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     int ix, iy, iz;
@@ -1248,6 +1289,7 @@ __global__ void __launch_bounds__(128) k_u2p_entropy(Grid G, Box b, U2PQueues Q,
 // finite.c:4599-4604, stores only the first NVMHD variables, and those
 // were not averaged for this kind), so a correction is only counted.
 __global__ void __launch_bounds__(128) k_u2p_rad(Grid G, Box b) {
+  after_previous();
   int ix, iy, iz, item;
   if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) return;
   if (polar_cell(G, iy)) return;   // corrected polar cells: field only (u2p.c:49-101)
@@ -1417,6 +1459,7 @@ __device__ inline void fixup_cell(const Grid &G, int ix, int iy, int iz, int *fi
   fixmark[c] = 1;
 }
 __global__ void k_fixup(Grid G, Box b, U2PQueues Q, int *fixmark) {
+  after_previous();
   const int n = Q.n[3];
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     int ix, iy, iz;
@@ -1428,6 +1471,7 @@ __global__ void k_fixup(Grid G, Box b, U2PQueues Q, int *fixmark) {
 // Applies the fixups of the queued cells and empties the queues of the stage.
 // The last block to finish empties the fixup queue itself.
 __global__ void k_commit(Grid G, Box b, U2PQueues Q, const int *fixmark) {
+  after_previous();
   if (blockIdx.x == 0 && (threadIdx.x < 3 || threadIdx.x == 4)) Q.n[threadIdx.x] = 0;
   const int n = *(volatile int *)(Q.n + 3);
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
@@ -1452,6 +1496,7 @@ __global__ void k_commit(Grid G, Box b, U2PQueues Q, const int *fixmark) {
 }
 // The end of an RK2 step: u = ut0 + (u - ut1) (addi_u pair of ko.c:614-615)
 __global__ void k_combine(Grid G, Box b) {
+  after_previous();
   int ix, iy, iz, item;
   if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) return;
   const long c = cell_index(G, ix, iy, iz);
@@ -1464,6 +1509,7 @@ __global__ void k_combine(Grid G, Box b) {
 }
 
 __global__ void k_begin_step(Grid G) {
+  after_previous();
   G.scal[S_DT] = 1. / G.scal[S_TSTEPDENMAX];
   G.scal[S_TSTEPDENMAX] = -1.;
 }
@@ -1704,35 +1750,37 @@ bool kgpu_rad_opts_valid(const kgpu_rad_solver_opts &o);
 template <int D>
 static void launch_flux(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b) {
   switch (mb) {
-    case 5: k_flux<D, 5><<<nb, 128, 0, st>>>(G, b, nullptr, nullptr); break;
-    case 6: k_flux<D, 6><<<nb, 128, 0, st>>>(G, b, nullptr, nullptr); break;
-    case 8: k_flux<D, 8><<<nb, 128, 0, st>>>(G, b, nullptr, nullptr); break;
-    default: k_flux<D, 7><<<nb, 128, 0, st>>>(G, b, nullptr, nullptr); break;
+    case 5: launch_next(st, nb, 128, k_flux<D, 5>, G, b, nullptr, nullptr); break;
+    case 6: launch_next(st, nb, 128, k_flux<D, 6>, G, b, nullptr, nullptr); break;
+    case 8: launch_next(st, nb, 128, k_flux<D, 8>, G, b, nullptr, nullptr); break;
+    default: launch_next(st, nb, 128, k_flux<D, 7>, G, b, nullptr, nullptr); break;
   }
 }
 template <int D>
 static void launch_flux_split(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b, const double *sl,
                               const double *sr) {
   switch (mb) {
-    case 5: k_flux<D, 5, true><<<nb, 128, 0, st>>>(G, b, sl, sr); break;
-    case 6: k_flux<D, 6, true><<<nb, 128, 0, st>>>(G, b, sl, sr); break;
-    case 8: k_flux<D, 8, true><<<nb, 128, 0, st>>>(G, b, sl, sr); break;
-    default: k_flux<D, 7, true><<<nb, 128, 0, st>>>(G, b, sl, sr); break;
+    case 5: launch_next(st, nb, 128, k_flux<D, 5, true>, G, b, sl, sr); break;
+    case 6: launch_next(st, nb, 128, k_flux<D, 6, true>, G, b, sl, sr); break;
+    case 8: launch_next(st, nb, 128, k_flux<D, 8, true>, G, b, sl, sr); break;
+    default: launch_next(st, nb, 128, k_flux<D, 7, true>, G, b, sl, sr); break;
   }
 }
 static void launch_update(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b, const double *dtp, double fac,
                           double *save) {
   switch (mb) {
-    case 3: k_update<3><<<nb, 128, 0, st>>>(G, b, dtp, fac, save); break;
-    case 5: k_update<5><<<nb, 128, 0, st>>>(G, b, dtp, fac, save); break;
-    default: k_update<4><<<nb, 128, 0, st>>>(G, b, dtp, fac, save); break;
+    case 2: launch_next(st, nb, 128, k_update<2>, G, b, dtp, fac, save); break;
+    case 3: launch_next(st, nb, 128, k_update<3>, G, b, dtp, fac, save); break;
+    case 5: launch_next(st, nb, 128, k_update<5>, G, b, dtp, fac, save); break;
+    default: launch_next(st, nb, 128, k_update<4>, G, b, dtp, fac, save); break;
   }
 }
 static void launch_u2p_first(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b, U2PQueues Q, int stop) {
   switch (mb) {
-    case 4: k_u2p<4><<<nb, 128, 0, st>>>(G, b, Q, stop); break;
-    case 6: k_u2p<6><<<nb, 128, 0, st>>>(G, b, Q, stop); break;
-    default: k_u2p<5><<<nb, 128, 0, st>>>(G, b, Q, stop); break;
+    case 2: launch_next(st, nb, 128, k_u2p<2>, G, b, Q, stop); break;
+    case 4: launch_next(st, nb, 128, k_u2p<4>, G, b, Q, stop); break;
+    case 6: launch_next(st, nb, 128, k_u2p<6>, G, b, Q, stop); break;
+    default: launch_next(st, nb, 128, k_u2p<5>, G, b, Q, stop); break;
   }
 }
 static bool tuning_valid(const kgpu_tuning &t) {
@@ -2326,9 +2374,16 @@ extern "C" int kgpu_read_restart(kgpu_ctx *c, const char *folder, int nout1, dou
 static int launch_bc(kgpu_ctx *c) {
   Grid &G = c->G;
   const BcParts P = bc_parts(G);
-  { LaunchScope ls(c, K_BC); k_bc<<<nblocks(P.total(), 128), 128, 0, c->stream>>>(G, P); }
+  { LaunchScope ls(c, K_BC); launch_next(c->stream, nblocks(P.total(), 128), 128, k_bc, G, P); }
   CKL("k_bc");
   return 0;
+}
+
+// two blocks per SM hold the whole box: a launch takes one thread's chain, so
+// the variants with the most registers run
+static bool small_grid(const kgpu_ctx *c, const Box &b, int per_block) {
+  const dim3 g = tile_grid(b, per_block);
+  return g.x * g.y <= 2u * (unsigned)c->sm_count;
 }
 
 static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *save) {
@@ -2337,7 +2392,7 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
   const int lim = G.int_order == 4 ? 2 : 1;
   int lx = G.nx > 1 ? lim : 0, ly = G.ny > 1 ? lim : 0, lz = G.nz > 1 ? lim : 0;
   Box wb{-lx, -ly, -lz, G.nx + 2 * lx, G.ny + 2 * ly, G.nz + 2 * lz};
-  { LaunchScope ls(c, K_WAVESPEEDS); k_wavespeeds<<<tile_grid(wb, 128), 128, 0, c->stream>>>(G, wb); }
+  { LaunchScope ls(c, K_WAVESPEEDS); launch_next(c->stream, tile_grid(wb, 128), 128, k_wavespeeds, G, wb); }
   CKL("k_wavespeeds");
   int ey0 = G.ny > 1 ? -1 : 0, eny = G.ny > 1 ? G.ny + 2 : 1;
   int ez0 = G.nz > 1 ? -1 : 0, enz = G.nz > 1 ? G.nz + 2 : 1;
@@ -2360,10 +2415,10 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
   // shows the directions apart.
   const bool together = !c->flux_split && !c->profiling && nall <= 16u * (unsigned)c->sm_count;
   if (together) {
-    { LaunchScope ls(c, K_FLUX0); k_flux_all<<<nall, 128, 0, c->stream>>>(G, F); }
+    { LaunchScope ls(c, K_FLUX0); launch_next(c->stream, nall, 128, k_flux_all, G, F); }
     CKL("k_flux_all");
     if (G.rad) {
-      { LaunchScope ls(c, K_FLUXRAD0); k_flux_rad_all<<<nall, 128, 0, c->stream>>>(G, F); }
+      { LaunchScope ls(c, K_FLUXRAD0); launch_next(c->stream, nall, 128, k_flux_rad_all, G, F); }
       CKL("k_flux_rad_all");
     }
   } else {
@@ -2372,13 +2427,13 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     const Box b = F.b[D];                                                                                             \
     if (c->flux_split) {                                                                                              \
       { LaunchScope ls(c, K_RECON0 + D);                                                                              \
-        k_recon<D><<<nblocks(b.n() * NVMAX, 256), 256, 0, c->stream>>>(G, b, c->fsl, c->fsr); }                        \
+        launch_next(c->stream, nblocks(b.n() * NVMAX, 256), 256, k_recon<D>, G, b, c->fsl, c->fsr); }                        \
       CKL("k_recon");                                                                                                 \
       LaunchScope ls(c, K_FLUX0 + D);                                                                                 \
       launch_flux_split<D>(c->flux_blocks, tile_grid(b, 64), c->stream, G, b, c->fsl, c->fsr);                         \
       CKL("k_flux");                                                                                                  \
       c->launches++;                                                                                                  \
-      k_flux_fix<D><<<2 * c->sm_count, 128, 0, c->stream>>>(G, b, c->fsl, c->fsr);                                     \
+      launch_next(c->stream, 2 * c->sm_count, 128, k_flux_fix<D>, G, b, c->fsl, c->fsr);                                     \
       CKL("k_flux_fix");                                                                                              \
     } else {                                                                                                          \
       LaunchScope ls(c, K_FLUX0 + D);                                                                                 \
@@ -2387,7 +2442,7 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     }                                                                                                                 \
     if (G.rad) {                                                                                                      \
       LaunchScope ls(c, K_FLUXRAD0 + D);                                                                              \
-      k_flux_rad<D><<<tile_grid(b, 64), 128, 0, c->stream>>>(G, b);                                                    \
+      launch_next(c->stream, tile_grid(b, 64), 128, k_flux_rad<D>, G, b);                                                    \
       CKL("k_flux_rad");                                                                                              \
     }                                                                                                                 \
   }
@@ -2399,21 +2454,21 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
   if (!c->flux_split) {
     // two blocks per SM loop over the queues
     LaunchScope ls(c, K_FLUX_FIX);
-    k_flux_fix_all<<<2 * c->sm_count, 128, 0, c->stream>>>(G, F);
+    launch_next(c->stream, 2 * c->sm_count, 128, k_flux_fix_all, G, F);
     CKL("k_flux_fix_all");
   }
   Box eb{0, 0, 0, G.nx + 1, G.ny + 1, G.nz + 1};
-  { LaunchScope ls(c, K_EMF); k_emf<<<nblocks(eb.n(), 128), 128, 0, c->stream>>>(G, eb); }
+  { LaunchScope ls(c, K_EMF); launch_next(c->stream, nblocks(eb.n(), 128), 128, k_emf, G, eb); }
   CKL("k_emf");
   if (G.polar_emf) {
     { LaunchScope ls(c, K_EMF); k_emf_polar<<<nblocks(2L * (G.nx + 1) * (G.nz + 1), 128), 128, 0, c->stream>>>(G); }
     CKL("k_emf_polar");
   }
   Box db = domain_box(G);
-  { LaunchScope ls(c, K_UPDATE); launch_update(c->update_blocks, tile_grid(db, 128), c->stream, G, db, dtp, fac, save); }
+  { LaunchScope ls(c, K_UPDATE); launch_update(small_grid(c, db, 128) ? 2 : c->update_blocks, tile_grid(db, 128), c->stream, G, db, dtp, fac, save); }
   CKL("k_update");
   if (G.rad) {
-    { LaunchScope ls(c, K_UPDATE_RAD); k_update_rad<<<tile_grid(db, 128), 128, 0, c->stream>>>(G, db, dtp, fac); }
+    { LaunchScope ls(c, K_UPDATE_RAD); launch_next(c->stream, tile_grid(db, 128), 128, k_update_rad, G, db, dtp, fac); }
     CKL("k_update_rad");
   }
   return 0;
@@ -2423,24 +2478,24 @@ static int launch_u2p(kgpu_ctx *c, int combine) {
   Grid &G = c->G;
   Box db = domain_box(G);
   const int sweep = c->sm_count * 4;   // grid of the queue passes (grid-stride loops)
-  { LaunchScope ls(c, K_U2P); launch_u2p_first(c->u2p_blocks, tile_grid(db, 128), c->stream, G, db, c->u2pq, c->u2p_pass_iters); }
+  { LaunchScope ls(c, K_U2P); launch_u2p_first(small_grid(c, db, 128) ? 2 : c->u2p_blocks, tile_grid(db, 128), c->stream, G, db, c->u2pq, c->u2p_pass_iters); }
   CKL("k_u2p");
-  { LaunchScope ls(c, K_U2P_RESUME); k_u2p_resume<<<sweep, 128, 0, c->stream>>>(G, db, c->u2pq, 0); }
+  { LaunchScope ls(c, K_U2P_RESUME); launch_next(c->stream, sweep, 128, k_u2p_resume, G, db, c->u2pq, 0); }
   CKL("k_u2p_resume");
-  { LaunchScope ls(c, K_U2P_ENT); k_u2p_entropy<<<sweep, 128, 0, c->stream>>>(G, db, c->u2pq, c->u2p_pass_iters); }
+  { LaunchScope ls(c, K_U2P_ENT); launch_next(c->stream, sweep, 128, k_u2p_entropy, G, db, c->u2pq, c->u2p_pass_iters); }
   CKL("k_u2p_entropy");
-  { LaunchScope ls(c, K_U2P_RESUME_ENT); k_u2p_resume<<<sweep, 128, 0, c->stream>>>(G, db, c->u2pq, 1); }
+  { LaunchScope ls(c, K_U2P_RESUME_ENT); launch_next(c->stream, sweep, 128, k_u2p_resume, G, db, c->u2pq, 1); }
   CKL("k_u2p_resume_entropy");
   if (G.rad) {
-    { LaunchScope ls(c, K_U2P_RAD); k_u2p_rad<<<tile_grid(db, 128), 128, 0, c->stream>>>(G, db); }
+    { LaunchScope ls(c, K_U2P_RAD); launch_next(c->stream, tile_grid(db, 128), 128, k_u2p_rad, G, db); }
     CKL("k_u2p_rad");
   }
-  { LaunchScope ls(c, K_FIXUP); k_fixup<<<c->sm_count, 128, 0, c->stream>>>(G, db, c->u2pq, c->fixmark); }
+  { LaunchScope ls(c, K_FIXUP); launch_next(c->stream, c->sm_count, 128, k_fixup, G, db, c->u2pq, c->fixmark); }
   CKL("k_fixup");
-  { LaunchScope ls(c, K_COMMIT); k_commit<<<c->sm_count, 128, 0, c->stream>>>(G, db, c->u2pq, c->fixmark); }
+  { LaunchScope ls(c, K_COMMIT); launch_next(c->stream, c->sm_count, 128, k_commit, G, db, c->u2pq, c->fixmark); }
   CKL("k_commit");
   if (combine) {
-    { LaunchScope ls(c, K_COMMIT); k_combine<<<tile_grid(db, 128), 128, 0, c->stream>>>(G, db); }
+    { LaunchScope ls(c, K_COMMIT); launch_next(c->stream, tile_grid(db, 128), 128, k_combine, G, db); }
     CKL("k_combine");
   }
   return launch_bc(c);
@@ -2553,7 +2608,7 @@ extern "C" int kgpu_flux_ct(kgpu_ctx *c) {
   if (c->flux_ct_done) return KGPU_ESTATE;   // the EMFs come from the fluxes before the rewrite
   Grid &G = c->G;
   Box eb{0, 0, 0, G.nx + 1, G.ny + 1, G.nz + 1};
-  k_emf<<<nblocks(eb.n(), 128), 128, 0, c->stream>>>(G, eb);
+  launch_next(c->stream, nblocks(eb.n(), 128), 128, k_emf, G, eb);
   CKL("k_emf");
   if (G.polar_emf) {
     k_emf_polar<<<nblocks(2L * (G.nx + 1) * (G.nz + 1), 128), 128, 0, c->stream>>>(G);
@@ -2594,7 +2649,7 @@ extern "C" int kgpu_get_tstepdenmax(kgpu_ctx *c, double *out) {
 
 extern "C" int kgpu_begin_step(kgpu_ctx *c, double *dt_out) {
   if (!c) return KGPU_EINVAL;
-  k_begin_step<<<1, 1, 0, c->stream>>>(c->G);
+  launch_next(c->stream, 1, 1, k_begin_step, c->G);
   CKL("k_begin_step");
   if (dt_out) CK(cudaMemcpyAsync(dt_out, c->G.scal + S_DT, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -2643,7 +2698,7 @@ static int enqueue_avg(kgpu_ctx *c, const double *dtp) {
 static int enqueue_rk2(kgpu_ctx *c) {
   Grid &G = c->G;
   int r;
-  { LaunchScope ls(c, K_BEGIN); k_begin_step<<<1, 1, 0, c->stream>>>(G); }
+  { LaunchScope ls(c, K_BEGIN); launch_next(c->stream, 1, 1, k_begin_step, G); }
   CKL("k_begin_step");
   if (c->polar_flags) {
     // copyi_u(1.,u,ut0) before do_correct (ko.c:577-579): ut0 keeps the
@@ -2685,7 +2740,9 @@ static int run_graph(kgpu_ctx *c, int nsteps, int kind, int (*enqueue)(kgpu_ctx 
     c->profiling = false;
     long long before = c->launches;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    g_capturing = true;
     int r = enqueue(c);
+    g_capturing = false;
     c->graph_launches = c->launches - before;
     c->launches = before;
     c->profiling = prof;
@@ -2834,9 +2891,9 @@ static int enqueue_implicit(kgpu_ctx *c, const double *dtp, double fac) {
   { LaunchScope ls(c, K_IMP_SCATTER);
     k_imp_scatter<<<nblocks(db.n(), 128), 128, 0, c->stream>>>(G, db, c->u2pq, c->imp_ppo, c->imp_uuo, c->imp_status); }
   CKL("k_imp_scatter");
-  { LaunchScope ls(c, K_FIXUP); k_fixup<<<c->sm_count, 128, 0, c->stream>>>(G, db, c->u2pq, c->fixmark); }
+  { LaunchScope ls(c, K_FIXUP); launch_next(c->stream, c->sm_count, 128, k_fixup, G, db, c->u2pq, c->fixmark); }
   CKL("k_fixup");
-  { LaunchScope ls(c, K_COMMIT); k_commit<<<c->sm_count, 128, 0, c->stream>>>(G, db, c->u2pq, c->fixmark); }
+  { LaunchScope ls(c, K_COMMIT); launch_next(c->stream, c->sm_count, 128, k_commit, G, db, c->u2pq, c->fixmark); }
   CKL("k_commit");
   return 0;
 }
@@ -2849,7 +2906,7 @@ static int enqueue_rk2imex(kgpu_ctx *c) {
   Box db = domain_box(G);
   const unsigned nb = nblocks(db.n(), 128);
   int r;
-  { LaunchScope ls(c, K_BEGIN); k_begin_step<<<1, 1, 0, c->stream>>>(G); }
+  { LaunchScope ls(c, K_BEGIN); launch_next(c->stream, 1, 1, k_begin_step, G); }
   CKL("k_begin_step");
   CK(cudaMemcpyAsync(G.ut0, G.u, G.ncell * G.nv * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
   if ((r = enqueue_implicit(c, dtp, gam))) return r;                       // U(1) = implicit from U(n)
