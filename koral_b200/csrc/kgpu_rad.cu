@@ -445,6 +445,7 @@ __device__ __forceinline__ void quads_run(const RadParams &R, const Cell &C, con
   bool todo = false, minus = true;
   unsigned cin0 = 0, cin1 = 0;
   bool begin = false;   // the attempt starts with the next trip
+  bool odd = false;
   while (true) {
     // quads without a cell take the next ones of the list
     const unsigned need = look-- > 0 ? 0u : __ballot_sync(FULL, col == 0 && !have && !idle);
@@ -504,8 +505,14 @@ __device__ __forceinline__ void quads_run(const RadParams &R, const Cell &C, con
     __syncwarp();
     // the entropy equation is never solved in the fluid frame
     const ImpParams P{PRIM, FRAME == IMP_FF ? (int)IMP_ENERGY : imp_attempt(att, sw).eq, FRAME};
+    // On MHD primitives an iteration is two trips, so the cells of a warp take
+    // turns: Jacobian columns in the odd trips, trials and base evaluations
+    // in the even ones.  A trip then runs the code of one of them (radiative
+    // torus 128x64x32 156 -> 152 ms, 262144 cells 100 -> 98).
+    odd = !odd;
+    const bool turn = have && (PRIM != IMP_MHD || (phase == PH_JAC) == odd);
     // the input of this trip's evaluation
-    bool act = have && (phase != PH_JAC || todo);
+    bool act = turn && (phase != PH_JAC || todo);
     int rejected = 0;   // trials of this trip that are not evaluated
     double pin[NVR], uu[NVR], x[4] = {0., 0., 0., 0.};
     {
@@ -513,7 +520,8 @@ __device__ __forceinline__ void quads_run(const RadParams &R, const Cell &C, con
 #pragma unroll
       for (int i = 0; i < NVR; i++) pin[i] = from[i];
     }
-    if (phase == PH_BASE) {
+    if (!turn) {
+    } else if (phase == PH_BASE) {
       iter++;
     } else if (phase == PH_JAC) {
       const double del = imp_fd_step(R, col, minus ? -1. : 1., q.ppp[col + sh], rg.g);
@@ -557,14 +565,14 @@ __device__ __forceinline__ void quads_run(const RadParams &R, const Cell &C, con
       if (i) x[i] = xi;
       else x[0] = xi;
     }
-    if (phase == PH_DAMP) {
+    if (turn && phase == PH_DAMP) {
 #pragma unroll
       for (int i = 0; i < 4; i++) pin[i + sh] = x[i];
     }
     const bool spent = rejected > 0 && !(xiapp >= R.maxdamping);   // no trial is left
     if (spent) act = false;
     __syncwarp();   // every lane has read the iterate
-    if (phase == PH_BASE) {
+    if (turn && phase == PH_BASE) {
 #pragma unroll
       for (int i = 0; i < NVR; i++)
         if ((i & 3) == col) q.ppp[i] = pin[i];
@@ -575,7 +583,7 @@ __device__ __forceinline__ void quads_run(const RadParams &R, const Cell &C, con
     if (PRIM == IMP_MHD) {
       if (act) {
         imp_rho_from_velocity(q.uu0, pin, rg.g);
-        imp_conserved(R, PRIM, q.uu0, pin, uu, rg);
+        imp_conserved(R, PRIM, q.uu0, pin, uu, rg, P.eq == IMP_ENTROPY);
       }
       together();
       if (act) u2pret = u2p_rad(R, uu, pin, rg, corr);
@@ -629,7 +637,7 @@ __device__ __forceinline__ void quads_run(const RadParams &R, const Cell &C, con
     }
     // a trial: kept or damped further (see imp_advance)
     bool fail = false, resid = act, chained = false;
-    if (have && phase == PH_DAMP && (spent || (PRIM == IMP_MHD && rejected > 0 && u2pret < 0))) {
+    if (turn && phase == PH_DAMP && (spent || (PRIM == IMP_MHD && rejected > 0 && u2pret < 0))) {
       resid = false;
       if (spent) {
         fail = true;
@@ -638,7 +646,7 @@ __device__ __forceinline__ void quads_run(const RadParams &R, const Cell &C, con
         xiapp = 1.;
         careful = true;
       }
-    } else if (have && phase == PH_DAMP) {
+    } else if (turn && phase == PH_DAMP) {
       if (col == 0) {
         st[3] += 1 + rejected;
         st[4] += in0;
@@ -824,14 +832,23 @@ __device__ __forceinline__ void quads_run(const RadParams &R, const Cell &C, con
 // barriers.  262144 cells of the batched-solve distribution, of which a fifth
 // runs through several attempts, from the cell's own guess / the network's:
 // warps running free 162 / 216 ms, in step in blocks of 4 warps 117 / 162 ms,
-// of 8 104 / 123 ms, of 16 112 / 106 ms.  With one cell a warp there is
-// little to share and much to wait for (1537 cells: 16 ms free, 18 in step),
-// so such a block runs free.
+// of 8 104 / 123 ms, of 16 112 / 106 ms.  A batch of no more cells than warps
+// has little to share and much to wait for (1537 cells: 16 ms free, 18 in
+// step), so there the warps run free (lock = false); letting single blocks of
+// a larger batch run free while their list is short cost it more than it gave
+// (20000 cells: 43 against 35 ms).
+//
+// Tried: one lane per cell, 7 warps of 32 cells an SM, for the bulk of a large
+// batch (every lane evaluates something of its own in every trip), handing
+// over to this form at the end: 127 against 114 ms for 262144 cells, 194
+// against 156 for the radiative torus: a warp waits for the slowest of 32
+// nested inversions, and the fetch-bound issue rate is the same.
 //
 // Before (passes over queues of cells, one lane a cell, a launch per pass and
 // for the cells that need whole warps): 363 / 288 ms, and 23 ms for 1537.
 __global__ void __launch_bounds__(32 * QUAD_WARPS, QUAD_BLOCKS)
-    k_rad_quads(RadParams R, Cell C, Work W, QuadLists Q, int *sm_role, int sms, unsigned cap, int warm_attempts) {
+    k_rad_quads(RadParams R, Cell C, Work W, QuadLists Q, int *sm_role, int sms, bool lock, unsigned cap,
+                int warm_attempts) {
   extern __shared__ __align__(16) unsigned char quad_smem[];
   QuadCell (*cells)[QUAD_CELLS] = reinterpret_cast<QuadCell(*)[QUAD_CELLS]>(quad_smem);
   __shared__ int choice[2];
@@ -869,10 +886,10 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, QUAD_BLOCKS)
     __syncthreads();
     const int r = choice[0], per = choice[1];
     if (r < 0) break;
-    if (r == 0) quads_run<IMP_RAD, IMP_LAB>(R, C, W, Q, cells[wib], per, per > 1, cap, warm_attempts, st);
-    else if (r == 1) quads_run<IMP_MHD, IMP_LAB>(R, C, W, Q, cells[wib], per, per > 1, cap, warm_attempts, st);
-    else if (r == 2) quads_run<IMP_RAD, IMP_FF>(R, C, W, Q, cells[wib], per, per > 1, cap, warm_attempts, st);
-    else quads_run<IMP_MHD, IMP_FF>(R, C, W, Q, cells[wib], per, per > 1, cap, warm_attempts, st);
+    if (r == 0) quads_run<IMP_RAD, IMP_LAB>(R, C, W, Q, cells[wib], per, lock, cap, warm_attempts, st);
+    else if (r == 1) quads_run<IMP_MHD, IMP_LAB>(R, C, W, Q, cells[wib], per, lock, cap, warm_attempts, st);
+    else if (r == 2) quads_run<IMP_RAD, IMP_FF>(R, C, W, Q, cells[wib], per, lock, cap, warm_attempts, st);
+    else quads_run<IMP_MHD, IMP_FF>(R, C, W, Q, cells[wib], per, lock, cap, warm_attempts, st);
   }
   for (int i = 0; i < 7; i++)
     if (i != 1) warp_add(W.stats + i, st[i]);
@@ -1332,7 +1349,8 @@ static int rad_solve_device(int n, const kgpu_rad_params *rp, const double *uu, 
     const unsigned cap = o.inner_cap > 0 ? (unsigned)(o.inner_cap + 3) / 4u : 0u;
     constexpr int kQuadSmem = QUAD_WARPS * QUAD_CELLS * (int)sizeof(QuadCell);
     RCK(cudaFuncSetAttribute(k_rad_quads, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuadSmem));
-    k_rad_quads<<<sms * QUAD_BLOCKS, 32 * QUAD_WARPS, kQuadSmem, st>>>(R, C, W, Q, W.count + 64, sms, cap,
+    k_rad_quads<<<sms * QUAD_BLOCKS, 32 * QUAD_WARPS, kQuadSmem, st>>>(R, C, W, Q, W.count + 64, sms,
+                                                                      n > sms * QUAD_BLOCKS * QUAD_WARPS, cap,
                                                                       o.warm_attempts);
     RCK(cudaGetLastError());
     k_rad_outputs<<<(n + 127) / 128, 128, 0, st>>>(R, C, n);

@@ -436,13 +436,19 @@ KG_HD double rad_Sfromu(const RadParams &R, double rho, double u) { return calc_
 // Conserved state that goes with the primitives pp when the other
 // component takes the opposite change of energy-momentum (rad.c:140-198 and
 // 883-960)
+// (entropy = false: uu[ENTR], which the entropy equation's residual reads,
+// is not wanted; on MHD primitives that spares the radiation's conversion)
 KG_HD void imp_conserved(const RadParams &R, int prim, const double *uu0, const double *pp, double *uu,
-                         const RadGeom &rg) {
+                         const RadGeom &rg, bool entropy = true) {
   Grid G;
   G.gamma = R.gamma;
   G.nv = NVMAX;
-  p2u_rad_full(G, pp, uu, rg.g);
-  uu[ENTR] = uu0[ENTR] - (uu[EE0] - uu0[EE0]);
+  if (prim == IMP_RAD || entropy) {
+    p2u_rad_full(G, pp, uu, rg.g);
+    uu[ENTR] = uu0[ENTR] - (uu[EE0] - uu0[EE0]);
+  } else {
+    p2u_full(G, pp, uu, rg.g);
+  }
   if (prim == IMP_RAD) {
     uu[RHO] = uu0[RHO];
     uu[1] = uu0[1] - (uu[EE0] - uu0[EE0]);
