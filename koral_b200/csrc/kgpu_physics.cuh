@@ -922,6 +922,22 @@ KG_HD double DM4(double W, double X, double Y, double Z) {
          dmin(dmin(fabs(W), fabs(X)), dmin(fabs(Y), fabs(Z)));
 }
 
+// The same two for finite arguments, bit for bit, by sign tests instead of
+// products of signs: arguments of one sign give that sign's smallest
+// magnitude, others a zero (negative where the product of signs is: DM4 with
+// W and X negative).  A negative zero counts as positive, as dsign has it.
+KG_HD double DMM_finite(double X, double Y) {
+  const bool nx = X < 0., ny = Y < 0.;
+  const double m = dmin(fabs(X), fabs(Y));
+  return nx != ny ? 0. : (nx ? -m : m);
+}
+KG_HD double DM4_finite(double W, double X, double Y, double Z) {
+  const bool nw = W < 0., nx = X < 0., ny = Y < 0., nz = Z < 0.;
+  double m = dmin(dmin(fabs(W), fabs(X)), dmin(fabs(Y), fabs(Z)));
+  if (nw != nx || nw != ny || nw != nz) m = 0.;
+  return nw && nx ? -m : m;
+}
+
 // PPM on a non-uniform grid (finite.c:142-225); returns the left (ul) and
 // right (ur) face values of the centre cell.
 KG_HD void ppm(double um2, double um1, double u0, double up1, double up2, double dxm2, double dxm1,
@@ -958,23 +974,41 @@ KG_HD void ppm(double um2, double um1, double u0, double up1, double up2, double
 
 // MP5 (finite.c:226-286), uniform spacing.  One face value: pass the
 // stencil in the direction of the face (a = far side, e = near side).
-KG_HD double mp5_face(double um2, double um1, double u0, double up1, double up2) {
+template <bool FINITE>
+KG_HD double mp5_limited(double um2, double um1, double u0, double up1, double up2, double VOR) {
   const double alpha = 4., epsm = 1.e-10, BB2 = 1.3333333;
-  double VOR = (3. * um2 - 20. * um1 + 90. * u0 + 60. * up1 - 5. * up2) / 128.;
-  double VMP = u0 + DMM(up1 - u0, alpha * (u0 - um1));
+  const double X = up1 - u0, Y = alpha * (u0 - um1);
+  double VMP = u0 + (FINITE ? DMM_finite(X, Y) : DMM(X, Y));
   if ((VOR - u0) * (VOR - VMP) < epsm) return VOR;
   double DJM1 = um2 - 2. * um1 + u0;
   double DJ = um1 - 2. * u0 + up1;
   double DJP1 = u0 - 2. * up1 + up2;
-  double DM4JPH = DM4(4. * DJ - DJP1, 4. * DJP1 - DJ, DJ, DJP1);
-  double DM4JMH = DM4(4. * DJ - DJM1, 4. * DJM1 - DJ, DJ, DJM1);
+  const double a = 4. * DJ - DJP1, b = 4. * DJP1 - DJ, c = 4. * DJ - DJM1, d = 4. * DJM1 - DJ;
+  double DM4JPH = FINITE ? DM4_finite(a, b, DJ, DJP1) : DM4(a, b, DJ, DJP1);
+  double DM4JMH = FINITE ? DM4_finite(c, d, DJ, DJM1) : DM4(c, d, DJ, DJM1);
   double VUL = u0 + alpha * (u0 - um1);
   double VAV = 0.5 * (u0 + up1);
   double VMD = VAV - 0.5 * DM4JPH;
   double VLC = u0 + 0.5 * (u0 - um1) + BB2 * DM4JMH;
   double VMIN = dmax(dmin(u0, dmin(up1, VMD)), dmin(u0, dmin(VUL, VLC)));
   double VMAX = dmin(dmax(u0, dmax(up1, VMD)), dmax(u0, dmax(VUL, VLC)));
-  return VOR + DMM(VMIN - VOR, VMAX - VOR);
+  return VOR + (FINITE ? DMM_finite(VMIN - VOR, VMAX - VOR) : DMM(VMIN - VOR, VMAX - VOR));
+}
+// the products of signs, for stencils with an infinity, a NaN or values near
+// the end of the range: out of line, they do not occur in a running flow
+static __host__ __device__ __noinline__ double mp5_any(double um2, double um1, double u0, double up1, double up2,
+                                                       double VOR) {
+  return mp5_limited<false>(um2, um1, u0, up1, up2, VOR);
+}
+// The face flux is bound by the issue of its instructions, and more than half
+// of them were MP5's: the products of signs took 40 of 60 floating-point
+// instructions of a limiter.  Per launch on the 192x96x64 torus: x 0.393 ->
+// 0.357 ms, y 0.381 -> 0.354, z 0.381 -> 0.359.
+KG_HD double mp5_face(double um2, double um1, double u0, double up1, double up2) {
+  double VOR = (3. * um2 - 20. * um1 + 90. * u0 + 60. * up1 - 5. * up2) / 128.;
+  // false for a NaN or an infinity among the values too
+  if (!(fabs(um2) + fabs(um1) + fabs(u0) + fabs(up1) + fabs(up2) < 1.e300)) return mp5_any(um2, um1, u0, up1, up2, VOR);
+  return mp5_limited<true>(um2, um1, u0, up1, up2, VOR);
 }
 
 }  // namespace kgpu
