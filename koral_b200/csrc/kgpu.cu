@@ -856,14 +856,61 @@ __global__ void k_emf(Grid G, Box b) {
 // unsplit update with metric source terms (finite.c:1062-1160,
 // f_metric_source_term_arb physics.c:324-465)
 // ---------------------------------------------------------------------------
-template <int MB = KGPU_UPDATE_MIN_BLOCKS>
+// Bound by the latency of its ~190 loads a cell at 16 warps an SM.  SHARED: the
+// four planes of a tile read the same 64 Christoffel rows of an axisymmetric
+// metric, so the block copies each row once to shared memory (16 KB), and the
+// copies land while the stress tensor is formed; with one plane a block, or a
+// metric of its own for every plane, no two warps share a row and the kernel
+// loads them itself.  The conserved quantities and the left faces' fluxes are
+// needed last: their lines are fetched to L2 at the start (the right faces'
+// lines are the neighbours').  192x96x64: 0.346 ms, rows shared 0.331, lines
+// fetched 0.316, both 0.295; the EMFs fetched too 0.301 (they are in L2 from
+// the kernel before).  A grid whose blocks all run at once (MB = 2) has its
+// arrays in L2 and its loads in flight together, and does neither: 40 steps of
+// the 128x128 vortex 5.75 ms, 5.78 with the fetches.
+template <bool SHARED, int MB = KGPU_UPDATE_MIN_BLOCKS>
 __global__ void __launch_bounds__(128, MB) k_update(Grid G, Box b, const double *dtp, double fac,
                                                                         double *save) {
+  __shared__ double kr[SHARED ? 64 * 32 : 1];
   after_previous();
   int ix, iy, iz, item;
-  if (!tile_coord(b, 128, threadIdx.x, ix, iy, iz, item)) return;
+  const bool valid = tile_coord(b, 128, threadIdx.x, ix, iy, iz, item);
+  if (SHARED) {
+    const unsigned lane = threadIdx.x & 31, part = threadIdx.x >> 5;   // a quarter of the rows to each warp
+    const unsigned pl = blockIdx.x * 32u + lane;
+    if (pl < (unsigned)(b.nx * b.ny)) {
+      const unsigned r = pl / (unsigned)b.nx;
+      const double *K = G.gkr + met_index(G, b.x0 + (int)(pl - r * (unsigned)b.nx), b.y0 + (int)r, 0);
+      const unsigned to = (unsigned)__cvta_generic_to_shared(kr + lane);
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const int row = (int)part * 16 + i;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to + (unsigned)row * 256u),
+                     "l"(K + (long)row * G.nmet) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  if (!valid) {   // past the box's end: the first cell, up to the barrier
+    if (!SHARED) return;
+    ix = b.x0;
+    iy = b.y0;
+    iz = b.z0;
+  }
   constexpr int nv = NVMAX;
   const long c = cell_index(G, ix, iy, iz);
+  if (MB > 2) {   // fetch what the end of the kernel reads
+    const long fx = face_index(G, ix, iy, iz, 0), fy = face_index(G, ix, iy, iz, 1), fz = face_index(G, ix, iy, iz, 2);
+#define PF(a) asm volatile("prefetch.global.L2 [%0];" ::"l"(a))
+#pragma unroll
+    for (int iv = 0; iv < nv; iv++) {
+      PF(G.u + iv * G.ncell + c);
+      if (G.nx > 1 && iv < B1) PF(G.flb[0] + iv * G.nface[0] + fx);
+      if (G.ny > 1 && iv < B1) PF(G.flb[1] + iv * G.nface[1] + fy);
+      if (G.nz > 1 && iv < B1) PF(G.flb[2] + iv * G.nface[2] + fz);
+    }
+#undef PF
+  }
   const double dt = fac * dtp[0];
   double pp[NVMAX];
   load_cell(G.p, G.ncell, c, pp);
@@ -899,15 +946,28 @@ __global__ void __launch_bounds__(128, MB) k_update(Grid G, Box b, const double 
   {
     const long mi = met_index(G, ix, iy, iz);
     const double gdetu = g.gdet;
+    if (SHARED) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      if (!valid) return;
+    }
     double s1 = 0., s2 = 0., s3 = 0., s4 = 0.;
     for (int kk = 0; kk < 4; kk++)
       for (int l = 0; l < 4; l++) {
         double gt = gdetu * T[kk][l];
-        const double *K = G.gkr + (long)(l * 16 + kk) * G.nmet + mi;
-        s1 += gt * __ldg(K + 0 * 4 * G.nmet);
-        s2 += gt * __ldg(K + 1 * 4 * G.nmet);
-        s3 += gt * __ldg(K + 2 * 4 * G.nmet);
-        s4 += gt * __ldg(K + 3 * 4 * G.nmet);
+        if (SHARED) {
+          const double *K = kr + (l * 16 + kk) * 32 + (threadIdx.x & 31);
+          s1 += gt * K[0 * 128];
+          s2 += gt * K[1 * 128];
+          s3 += gt * K[2 * 128];
+          s4 += gt * K[3 * 128];
+        } else {
+          const double *K = G.gkr + (long)(l * 16 + kk) * G.nmet + mi;
+          s1 += gt * __ldg(K + 0 * 4 * G.nmet);
+          s2 += gt * __ldg(K + 1 * 4 * G.nmet);
+          s3 += gt * __ldg(K + 2 * 4 * G.nmet);
+          s4 += gt * __ldg(K + 3 * 4 * G.nmet);
+        }
       }
     ms[1] = s1; ms[2] = s2; ms[3] = s3; ms[4] = s4;
   }
@@ -1768,11 +1828,15 @@ static void launch_flux_split(int mb, dim3 nb, cudaStream_t st, const Grid &G, B
 }
 static void launch_update(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b, const double *dtp, double fac,
                           double *save) {
-  switch (mb) {
-    case 2: launch_next(st, nb, 128, k_update<2>, G, b, dtp, fac, save); break;
-    case 3: launch_next(st, nb, 128, k_update<3>, G, b, dtp, fac, save); break;
-    case 5: launch_next(st, nb, 128, k_update<5>, G, b, dtp, fac, save); break;
-    default: launch_next(st, nb, 128, k_update<4>, G, b, dtp, fac, save); break;
+  const bool shared = mb > 2 && G.axisym && b.nz >= 4;   // tiles of four planes of one metric
+  switch (mb + 8 * shared) {
+    case 2: launch_next(st, nb, 128, k_update<false, 2>, G, b, dtp, fac, save); break;
+    case 3: launch_next(st, nb, 128, k_update<false, 3>, G, b, dtp, fac, save); break;
+    case 4: launch_next(st, nb, 128, k_update<false, 4>, G, b, dtp, fac, save); break;
+    case 5: launch_next(st, nb, 128, k_update<false, 5>, G, b, dtp, fac, save); break;
+    case 11: launch_next(st, nb, 128, k_update<true, 3>, G, b, dtp, fac, save); break;
+    case 13: launch_next(st, nb, 128, k_update<true, 5>, G, b, dtp, fac, save); break;
+    default: launch_next(st, nb, 128, k_update<true, 4>, G, b, dtp, fac, save); break;
   }
 }
 static void launch_u2p_first(int mb, dim3 nb, cudaStream_t st, const Grid &G, Box b, U2PQueues Q, int stop) {
