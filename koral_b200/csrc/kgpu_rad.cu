@@ -26,11 +26,11 @@
 
 using namespace kgpu;
 
-// resident blocks of 128 threads per SM the solver kernels are compiled for
+// resident blocks of 128 threads per SM the one-lane-a-cell kernels (plain and
+// persistent forms) are compiled for
 // (128 registers at 4: on the settled 256x128x64 radiative torus 16 warps
 // per SM hide more of the solver's instruction-fetch and FP64 latency than
-// the added spills cost: 197 against 224 ms per step at 1 block, 201 at 5,
-// 203 at 6, with a tail of as many blocks; batched-solve cells within 5%)
+// the added spills cost)
 #ifndef KGPU_RAD_MIN_BLOCKS
 #define KGPU_RAD_MIN_BLOCKS 4
 #endif
@@ -133,10 +133,9 @@ struct Work {
   int *qs;          // cooperative queue of the current pass: cell indices ...
   ImpState *ss;     // ... and the states of their interrupted evaluations
   int nslots;       // its capacity
-  unsigned long long *stats;  // [0] Newton iterations, [1] passes, [2] fallbacks of the warm start,
+  unsigned long long *stats;  // [0] Newton iterations, [1] resident launches, [2] fallbacks of the warm start,
                               // [3] residual evaluations, [4] Newton steps of the nested MHD inversions,
                               // [5] their W-function evaluations, [6] evaluations handed to a warp
-  unsigned *tail_done;        // blocks of the running tail launch that have finished
   unsigned *ctl;              // persistent form: [0] next work-list entry, [1] cells handed over paused
                               // (listed in q[1][0]), [2] next hand-over taken by k_rad_finish,
                               // [3] evaluations handed over with their state (qs/ss)
@@ -168,7 +167,6 @@ size_t work_layout(int n, Work *w, char *base) {
     }
   p = take((size_t)kCounters * 4); if (w) w->count = (int *)p;
   p = take(8 * sizeof(unsigned long long)); if (w) w->stats = (unsigned long long *)p;
-  p = take(sizeof(unsigned)); if (w) w->tail_done = (unsigned *)p;
   p = take(4 * sizeof(unsigned)); if (w) w->ctl = (unsigned *)p;
   const int slots = slow_slots(n);
   p = take((size_t)slots * 4); if (w) w->qs = (int *)p;
@@ -1316,7 +1314,6 @@ static int rad_solve_device(int n, const kgpu_rad_params *rp, const double *uu, 
   Work W;
   work_layout(n, &W, base);
   RCK(cudaMemsetAsync(W.count, 0, (size_t)kCounters * 4, st));
-  RCK(cudaMemsetAsync(W.tail_done, 0, sizeof(unsigned), st));
   RCK(cudaMemsetAsync(W.ctl, 0, 4 * sizeof(unsigned), st));
   if (acc) W.stats = acc;
   else RCK(cudaMemsetAsync(W.stats, 0, 8 * sizeof(unsigned long long), st));
