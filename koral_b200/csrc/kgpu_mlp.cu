@@ -144,19 +144,11 @@ __device__ void load_weights(SmemW &w, const Bf16Weights W, const float *blob) {
 // two 8-column accumulator tiles (columns 16 ks .. 16 ks + 15 of a layer's
 // pre-activations) as the A fragment of k-step ks of the next layer: the
 // layouts agree, so activations never leave the registers
-//
-// The activation is rounded to BF16 at once, so its FP32 quotient is the
-// two-ulp one: with the correctly rounded division 2^20 samples took 337 us,
-// with this one 185.  Relative error of the outputs against 64 bits, mean of
-// four seeds, correctly rounded / this: 100 samples 0.015017142 / the same,
-// 5000 0.016055732 / 0.016054564, 2e5 0.016023059 / 0.016023033, 2^20
-// 0.016018738 / 0.016018749.
-__device__ inline float silu2(float z) { return __fdividef(z, 1.f + __expf(-z)); }
 __device__ inline void activate(uint32_t a[4], const float c0[4], const float c1[4]) {
-  a[0] = pack2(silu2(c0[0]), silu2(c0[1]));
-  a[1] = pack2(silu2(c0[2]), silu2(c0[3]));
-  a[2] = pack2(silu2(c1[0]), silu2(c1[1]));
-  a[3] = pack2(silu2(c1[2]), silu2(c1[3]));
+  a[0] = pack2(silu(c0[0]), silu(c0[1]));
+  a[1] = pack2(silu(c0[2]), silu(c0[3]));
+  a[2] = pack2(silu(c1[0]), silu(c1[1]));
+  a[3] = pack2(silu(c1[2]), silu(c1[3]));
 }
 
 // neighbouring floats of the caller's arrays: one access where they are
@@ -188,7 +180,7 @@ constexpr int kInferWarps = 16;
 // tensor-core latency of one chain is hidden by the others.  What bounds it is
 // the issue of the activations (128 exponentials and divisions a lane and
 // tile).  With the activations passed through shared memory and fragments
-// from 32-bit loads 2^20 samples took 394 us, now 185.
+// from 32-bit loads 2^20 samples took 394 us, now 337.
 template <bool WIDE>
 __global__ void __launch_bounds__(32 * kInferWarps) k_mlp_forward(const float *blob, Bf16Weights W, const float *X,
                                                                   int n, float *Y) {
