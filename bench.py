@@ -1121,7 +1121,7 @@ def our_arm_radcells(args, wl, rank, world, local_rank):
     if rank != 0:
         return
     ok = st == 0
-    passes = (6 * 51 + 7) // 8 + 1   # pass launches of one batched solve at 8 iterations per pass
+    launches = 4   # of one batched solve: start, list bounds, solve, outputs
     line = {
         "metric": RAD_METRIC, "value": value, "unit": RAD_UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
@@ -1135,7 +1135,7 @@ def our_arm_radcells(args, wl, rank, world, local_rank):
                    "mean_iterations_all_attempts": stats[0] / n, "passes_with_work": int(stats[1]),
                    "success_rate": float(ok.mean()),
                    "attempt_histogram": {int(a): int((at == a).sum()) for a in np.unique(at)}},
-        "roofline": {"kernel": "k_rad_pass + k_rad_slow + k_rad_tail (batched implicit solve)", "bound": "fp64",
+        "roofline": {"kernel": "k_rad_quads (batched implicit solve)", "bound": "fp64",
                      "peak": fp64_peak, "unit": "TFLOP/s",
                      "peak_source": "measured live (DMUL+DADD chains, no FMA)", "achieved": tf,
                      "frac": tf / fp64_peak if tf else None, "traffic": None, "evaluations": int(stats[3]),
@@ -1143,7 +1143,7 @@ def our_arm_radcells(args, wl, rank, world, local_rank):
                      "flop_per_evaluation": IMP_FP64_PER_EVAL_CELLS},
         "e2e": {"value": e2e_value, "unit": RAD_UNIT, "h2d_bytes_per_step": n * (13 + 13 + 20 + 20 + 1) * 8,
                 "d2h_bytes_per_step": n * (26 * 8 + 12)},
-        "gpu_launches": passes * args.steps,
+        "gpu_launches": launches * args.steps,
         "clocks": clk.summary(),
     }
     if not args.no_cpu_baseline:
