@@ -41,7 +41,11 @@ using namespace kgpu;
 // error plumbing
 // ---------------------------------------------------------------------------
 static thread_local char g_lasterr[256] = "";
+// The runtime keeps the error of a failed call (an allocation that did not
+// fit, say) until it is asked for; the next launch's check would report it as
+// its own and leave its stage half done, its work queues and flags set.
 static int set_err(const char *what, cudaError_t e) {
+  (void)cudaGetLastError();
   snprintf(g_lasterr, sizeof(g_lasterr), "%s: %s", what, cudaGetErrorString(e));
   return KGPU_ECUDA;
 }

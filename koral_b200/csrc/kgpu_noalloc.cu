@@ -207,6 +207,7 @@ extern "C" int kgpu_u2p_cells_static(int n, const kgpu_config *cfg, const double
   do {                                                                               \
     e = (call);                                                                      \
     if (e != cudaSuccess) {                                                          \
+      (void)cudaGetLastError(); /* not left for the next launch's check */           \
       snprintf(g_err, sizeof(g_err), "%s: %s", #call, cudaGetErrorString(e));        \
       return KGPU_ECUDA;                                                             \
     }                                                                                \
