@@ -22,10 +22,9 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
-#include <map>
-
 #include "../../include/koral_b200.h"
 #include "kgpu_mlp.cuh"
+#include "kgpu_slots.h"
 
 using namespace kgpu;
 
@@ -387,26 +386,47 @@ bool params_of(const kgpu_config *cfg, int nv, U2PParams &P) {
   return true;
 }
 
-// The counters of a call that reports them: one small buffer per host thread
-// and device, free again when the call has synchronised, given back when the
-// thread ends.  (A stream-ordered allocation went back to the driver at every
-// synchronisation, and mapping it anew cost a few hundred microseconds.)
-struct ThreadCounters {
-  std::map<int, unsigned long long *> of_device;
-  ~ThreadCounters() {
-    for (auto &kv : of_device) cudaFree(kv.second);
+// The counters of a call that reports them: a row of an array of the module,
+// held from the call's start until its stream has been synchronised.  The
+// array belongs to the device's context and its address is asked for in every
+// call, so no device pointer outlives what it points to.  With every row held
+// by other threads' calls the call allocates its own, as all did at first: a
+// stream-ordered allocation goes back to the driver at every synchronisation,
+// and mapping it anew costs a few hundred microseconds.
+__device__ unsigned long long g_counters[Slots::N][3];
+Slots g_counter_rows;
+
+class CallCounters {
+ public:
+  explicit CallCounters(cudaStream_t s) : s_(s) {}
+  ~CallCounters() {
+    if (row_ < 0 && !p_) return;
+    if (!synced_) cudaStreamSynchronize(s_);   // a call that failed: what it enqueued may still run
+    if (row_ >= 0) g_counter_rows.give(row_);
+    else cudaFreeAsync(p_, s_);
   }
+  // cleared on the stream
+  cudaError_t open(unsigned long long **p) {
+    cudaError_t e;
+    row_ = g_counter_rows.take();
+    if (row_ >= 0) {
+      void *base = nullptr;
+      if ((e = cudaGetSymbolAddress(&base, g_counters)) != cudaSuccess) return e;
+      *p = (unsigned long long *)base + 3 * row_;
+    } else {
+      if ((e = cudaMallocAsync(&p_, 3 * sizeof(unsigned long long), s_)) != cudaSuccess) return e;
+      *p = (unsigned long long *)p_;
+    }
+    return cudaMemsetAsync(*p, 0, 3 * sizeof(unsigned long long), s_);
+  }
+  void synced() { synced_ = true; }
+
+ private:
+  cudaStream_t s_;
+  int row_ = -1;
+  void *p_ = nullptr;
+  bool synced_ = false;
 };
-cudaError_t thread_counters(unsigned long long **p) {
-  static thread_local ThreadCounters mine;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  unsigned long long *&q = mine.of_device[dev];
-  if (!q && (e = cudaMalloc(&q, 3 * sizeof(unsigned long long))) != cudaSuccess) return e;
-  *p = q;
-  return cudaSuccess;
-}
 
 }  // namespace
 
@@ -443,10 +463,8 @@ extern "C" int kgpu_u2p_cells_device(int n, const kgpu_config *cfg, int nv, cons
   if (n == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   unsigned long long *dstats = nullptr;
-  if (nstats > 0) {
-    WCK(thread_counters(&dstats));
-    WCK(cudaMemsetAsync(dstats, 0, 3 * sizeof(unsigned long long), s));
-  }
+  CallCounters counters(s);
+  if (nstats > 0) WCK(counters.open(&dstats));
   cudaError_t e;
   if (ypred) {
     k_u2p_warm_cells<<<(n + 127) / 128, 128, 0, s>>>(P, n, nv, uu, pp, g, G, ypred, wgate, sgate, status, fixup, iters,
@@ -468,7 +486,7 @@ extern "C" int kgpu_u2p_cells_device(int n, const kgpu_config *cfg, int nv, cons
   if (dstats) {
     unsigned long long h[3] = {0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, dstats, sizeof(h), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && (e = cudaStreamSynchronize(s)) == cudaSuccess) counters.synced();
     for (int k = 0; k < nstats; k++) stats[k] = h[k];
   }
   WCK(e);
