@@ -590,12 +590,17 @@ int kgpu_set_warm_gate(kgpu_ctx *ctx, int iters);
  * in the registers they are compiled for, the solver settings in how work
  * is scheduled).
  *  flux_blocks     blocks of 128 threads per SM the face-flux kernels are
- *                  compiled for: 5..8 (default 7)
+ *                  compiled for: 5..8 (default 7).  Without effect where
+ *                  the three directions run as one launch: face states
+ *                  reconstructed inside it, no more than 16 blocks per SM
+ *                  in all
  *  flux_split      1: the face states are reconstructed by a kernel of
  *                  their own (one thread per face and variable) and read by
  *                  the flux kernel; 0 (default): reconstructed inside it
  *  update_blocks   the same for the update kernel: 3..5 (default 4)
- *  u2p_blocks      the same for the first inversion pass: 4..6 (default 5)
+ *  u2p_blocks      the same for the first inversion pass: 4..6 (default 5).
+ *                  Both without effect on a grid of at most two blocks per
+ *                  SM, which runs the variants with the most registers
  *  u2p_pass_iters  Newton steps of the first inversion pass before a solve
  *                  is queued for resumption (default 8)
  *  implicit_mode   solver of op_implicit (KGPU_RAD_*; default batched)
@@ -620,14 +625,15 @@ int kgpu_set_tuning(kgpu_ctx *ctx, const kgpu_tuning *t);
  * whole time steps (RK2, or RK2IMEX with radiation) from the stream and
  * times them with CUDA events; the state, the time step and the counters
  * are restored afterwards, and the choice is applied.  Candidates: the
- * fused or split face flux, flux 5..8, update 3..5, u2p 4..6 blocks; u2p_pass_iters 4, 8, 16; with
- * radiation the batched and the persistent solver, inner_cap 32, 64, 128 and,
- * persistent, thin 4, 8, 16.  A candidate
- * replaces the incumbent only when it is faster by min_gain (a fraction,
- * e.g. 0.02) in the same round of trials.  The choice is cached per device
- * and grid configuration for the process: with reuse = 1 a cached choice
- * is applied without trials.  Outputs (optional): the chosen tuning and
- * the time per step of the starting and of the chosen tuning (ms[2]). */
+ * fused or split face flux; flux 5..8, update 3..5, u2p 4..6 blocks, where
+ * they have an effect (else the field stays as it is); u2p_pass_iters 4, 8,
+ * 16; with radiation the batched and the persistent solver, inner_cap 32, 64,
+ * 128 and, persistent, thin 4, 8, 16.  A candidate replaces the incumbent
+ * only when it is faster by min_gain (a fraction, e.g. 0.02) in the same
+ * round of trials.  The choice is cached per device and grid configuration
+ * for the process: with reuse = 1 a cached choice is applied without trials.
+ * Outputs (optional): the chosen tuning and the time per step of the starting
+ * and of the chosen tuning (ms[2]). */
 int kgpu_autotune(kgpu_ctx *ctx, int steps, double min_gain, int reuse, kgpu_tuning *chosen, double *ms);
 /* The autotuner's selection rule on its own: index of the fastest of n
  * timings if it beats timings[incumbent] by the fraction min_gain, else

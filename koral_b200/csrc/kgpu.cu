@@ -2454,17 +2454,12 @@ static bool small_grid(const kgpu_ctx *c, const Box &b, int per_block) {
   return g.x * g.y <= 2u * (unsigned)c->sm_count;
 }
 
-static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *save) {
-  Grid &G = c->G;
-  c->flux_ct_done = false;
-  const int lim = G.int_order == 4 ? 2 : 1;
-  int lx = G.nx > 1 ? lim : 0, ly = G.ny > 1 ? lim : 0, lz = G.nz > 1 ? lim : 0;
-  Box wb{-lx, -ly, -lz, G.nx + 2 * lx, G.ny + 2 * ly, G.nz + 2 * lz};
-  { LaunchScope ls(c, K_WAVESPEEDS); launch_next(c->stream, tile_grid(wb, 128), 128, k_wavespeeds, G, wb); }
-  CKL("k_wavespeeds");
-  int ey0 = G.ny > 1 ? -1 : 0, eny = G.ny > 1 ? G.ny + 2 : 1;
-  int ez0 = G.nz > 1 ? -1 : 0, enz = G.nz > 1 ? G.nz + 2 : 1;
-  int ex0 = -1, enx = G.nx + 2;
+// the face fluxes' boxes, one ring of cells wider than the domain across the
+// direction (none for a direction of one cell)
+static FaceBoxes face_boxes(const Grid &G) {
+  const int ey0 = G.ny > 1 ? -1 : 0, eny = G.ny > 1 ? G.ny + 2 : 1;
+  const int ez0 = G.nz > 1 ? -1 : 0, enz = G.nz > 1 ? G.nz + 2 : 1;
+  const int ex0 = -1, enx = G.nx + 2;
   FaceBoxes F{};
   F.b[0] = Box{0, ey0, ez0, G.nx > 1 ? G.nx + 1 : 0, eny, enz};
   F.b[1] = Box{ex0, 0, ez0, enx, G.ny > 1 ? G.ny + 1 : 0, enz};
@@ -2475,13 +2470,29 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
     F.gx[d] = g.x;
     F.n[d] = g.x * g.y;
   }
+  return F;
+}
+// One launch for the three directions while they fill the chip only a few
+// times: on the 128x128 vortex, 268 blocks a direction, a launch takes as
+// long as one thread's chain whatever it computes.  Larger grids lose
+// nothing to the launches and gain from k_flux's occupancy.
+static bool faces_in_one_launch(const kgpu_ctx *c, int split) {
+  const FaceBoxes F = face_boxes(c->G);
+  return !split && F.n[0] + F.n[1] + F.n[2] <= 16u * (unsigned)c->sm_count;
+}
+
+static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *save) {
+  Grid &G = c->G;
+  c->flux_ct_done = false;
+  const int lim = G.int_order == 4 ? 2 : 1;
+  int lx = G.nx > 1 ? lim : 0, ly = G.ny > 1 ? lim : 0, lz = G.nz > 1 ? lim : 0;
+  Box wb{-lx, -ly, -lz, G.nx + 2 * lx, G.ny + 2 * ly, G.nz + 2 * lz};
+  { LaunchScope ls(c, K_WAVESPEEDS); launch_next(c->stream, tile_grid(wb, 128), 128, k_wavespeeds, G, wb); }
+  CKL("k_wavespeeds");
+  const FaceBoxes F = face_boxes(G);
   const unsigned nall = F.n[0] + F.n[1] + F.n[2];
-  // One launch for the three directions while they fill the chip only a few
-  // times: on the 128x128 vortex, 268 blocks a direction, a launch takes as
-  // long as one thread's chain whatever it computes.  Larger grids lose
-  // nothing to the launches and gain from k_flux's occupancy.  A profiled step
-  // shows the directions apart.
-  const bool together = !c->flux_split && !c->profiling && nall <= 16u * (unsigned)c->sm_count;
+  // a profiled step shows the directions apart
+  const bool together = faces_in_one_launch(c, c->flux_split) && !c->profiling;
   if (together) {
     { LaunchScope ls(c, K_FLUX0); launch_next(c->stream, nall, 128, k_flux_all, G, F); }
     CKL("k_flux_all");
@@ -3116,6 +3127,7 @@ std::mutex g_tuned_mutex;
 struct Knob {
   int *(*field)(kgpu_tuning &);
   std::vector<int> values;
+  bool (*acts)(const kgpu_ctx *, const kgpu_tuning &) = nullptr;   // whether this grid's launches read it (none: they do)
 };
 }  // namespace
 
@@ -3182,11 +3194,15 @@ extern "C" int kgpu_autotune(kgpu_ctx *c, int steps, double min_gain, int reuse,
   cudaEvent_t ea, eb;
   CK(cudaEventCreate(&ea));
   CK(cudaEventCreate(&eb));
+  const auto not_small = [](const kgpu_ctx *x, const kgpu_tuning &) {
+    return !small_grid(x, domain_box(x->G), 128);
+  };
   std::vector<Knob> knobs = {
       {[](kgpu_tuning &t) { return &t.flux_split; }, {0, 1}},
-      {[](kgpu_tuning &t) { return &t.flux_blocks; }, {5, 6, 7, 8}},
-      {[](kgpu_tuning &t) { return &t.update_blocks; }, {3, 4, 5}},
-      {[](kgpu_tuning &t) { return &t.u2p_blocks; }, {4, 5, 6}},
+      {[](kgpu_tuning &t) { return &t.flux_blocks; }, {5, 6, 7, 8},
+       [](const kgpu_ctx *x, const kgpu_tuning &t) { return !faces_in_one_launch(x, t.flux_split); }},
+      {[](kgpu_tuning &t) { return &t.update_blocks; }, {3, 4, 5}, not_small},
+      {[](kgpu_tuning &t) { return &t.u2p_blocks; }, {4, 5, 6}, not_small},
       {[](kgpu_tuning &t) { return &t.u2p_pass_iters; }, {4, 8, 16}},
   };
   if (G.rad) {
@@ -3199,6 +3215,7 @@ extern "C" int kgpu_autotune(kgpu_ctx *c, int steps, double min_gain, int reuse,
   double ms_best = ms_start;
   int status = 0;
   for (size_t ki = 0; ki < knobs.size() && !status; ki++) {
+    if (knobs[ki].acts && !knobs[ki].acts(c, best)) continue;   // every candidate would be the same launch
     std::vector<Knob> round = {knobs[ki]};
     // the settings that belong to the solver form just chosen
     if (G.rad && knobs[ki].field(best) == &best.implicit.inner_cap) {

@@ -36,3 +36,19 @@ def test_autotune_torus_same_bits(kgpu):
 
 def test_autotune_radiative_torus_same_bits(kgpu):
     run_pair(kgpu, lambda: kgpu.radtorus(32, 16, 8), 3, True)
+
+
+def test_autotune_leaves_fields_without_effect(kgpu):
+    """On a grid whose launches do not read a field (the header says which)
+    its candidates are one and the same launch: the field stays as it is,
+    whatever the noise of the timings (min_gain 0)."""
+    s = kgpu.fm_torus(24, 16, 8)
+    s.rk2_steps(2)
+    d = s.tuning()
+    for _ in range(4):
+        t, _ = s.autotune(steps=2, min_gain=0.)
+        assert (t.update_blocks, t.u2p_blocks) == (d.update_blocks, d.u2p_blocks)
+        if t.flux_split == 0:
+            assert t.flux_blocks == d.flux_blocks
+        t.flux_split, t.flux_blocks = 0, d.flux_blocks
+        s.set_tuning(t)
