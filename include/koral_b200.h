@@ -315,9 +315,12 @@ const char *kgpu_u2p_cells_static_error(void);
 int kgpu_get_stream(kgpu_ctx *ctx, void **stream);
 /* When enabled, every launch outside a CUDA graph is bracketed by CUDA
  * events; kgpu_profile_read returns the summed device time and launch count
- * of one kernel kind (0 <= kernel < kgpu_num_kernels()) and its name.  The
- * face flux of a direction (k_flux_x/y/z) is timed and counted together
- * with its magnetic-floor pass, as one. */
+ * of one kernel kind (0 <= kernel < kgpu_num_kernels()) and its name.  A
+ * profiled step launches what any other step from the stream does.  The face
+ * flux is k_flux_x/y/z, a launch a direction, or on small grids k_flux_all
+ * (and the radiation's likewise); its magnetic-floor pass is k_flux_fix, one
+ * launch for all directions, but timed and counted with k_flux_x/y/z where
+ * the face states are reconstructed by a kernel of their own. */
 int kgpu_profile_enable(kgpu_ctx *ctx, int on);
 int kgpu_profile_read(kgpu_ctx *ctx, int kernel, double *total_ms, long long *count, const char **name);
 int kgpu_profile_reset(kgpu_ctx *ctx);

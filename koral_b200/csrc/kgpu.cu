@@ -1790,14 +1790,14 @@ __global__ void k_fill(double *a, long n, double v) {
 enum KernelId { K_BC = 0, K_WAVESPEEDS, K_FLUX0, K_FLUX1, K_FLUX2, K_EMF, K_UPDATE, K_U2P, K_U2P_RESUME,
                 K_U2P_ENT, K_U2P_RESUME_ENT, K_FIXUP, K_COMMIT, K_BEGIN, K_FLUXRAD0, K_FLUXRAD1, K_FLUXRAD2,
                 K_UPDATE_RAD, K_U2P_RAD, K_IMP_GATHER, K_IMP_WARM, K_IMP_SOLVE, K_IMP_SCATTER, K_IMEX, K_RECON0,
-                K_RECON1, K_RECON2, K_AVG, K_FLUX_FIX, K_NKERNELS };
+                K_RECON1, K_RECON2, K_AVG, K_FLUX_FIX, K_FLUX_ALL, K_FLUXRAD_ALL, K_NKERNELS };
 static const char *kKernelNames[K_NKERNELS] = {"k_bc", "k_wavespeeds", "k_flux_x", "k_flux_y", "k_flux_z", "k_emf",
                                                "k_update", "k_u2p", "k_u2p_resume", "k_u2p_entropy",
                                                "k_u2p_resume_entropy", "k_fixup", "k_commit", "k_begin_step",
                                                "k_flux_rad_x", "k_flux_rad_y", "k_flux_rad_z", "k_update_rad",
                                                "k_u2p_rad", "k_imp_gather", "k_imp_warm_start", "k_imp_solve",
                                                "k_imp_scatter", "k_imex", "k_recon_x", "k_recon_y", "k_recon_z",
-                                               "k_save_avg", "k_flux_fix"};
+                                               "k_save_avg", "k_flux_fix", "k_flux_all", "k_flux_rad_all"};
 
 int kgpu_rad_solve_enqueue(int n, const kgpu_rad_params *rp, const double *uu, const double *pp, const double *g,
                            const double *G, const double *dt, const float *ypred, double *pp_out, double *uu_out,
@@ -2491,13 +2491,12 @@ static int launch_explicit(kgpu_ctx *c, const double *dtp, double fac, double *s
   CKL("k_wavespeeds");
   const FaceBoxes F = face_boxes(G);
   const unsigned nall = F.n[0] + F.n[1] + F.n[2];
-  // a profiled step shows the directions apart
-  const bool together = faces_in_one_launch(c, c->flux_split) && !c->profiling;
+  const bool together = faces_in_one_launch(c, c->flux_split);
   if (together) {
-    { LaunchScope ls(c, K_FLUX0); launch_next(c->stream, nall, 128, k_flux_all, G, F); }
+    { LaunchScope ls(c, K_FLUX_ALL); launch_next(c->stream, nall, 128, k_flux_all, G, F); }
     CKL("k_flux_all");
     if (G.rad) {
-      { LaunchScope ls(c, K_FLUXRAD0); launch_next(c->stream, nall, 128, k_flux_rad_all, G, F); }
+      { LaunchScope ls(c, K_FLUXRAD_ALL); launch_next(c->stream, nall, 128, k_flux_rad_all, G, F); }
       CKL("k_flux_rad_all");
     }
   } else {
