@@ -81,11 +81,9 @@ RAD_METRIC = "implicit solves/s (1 B200)"
 
 # From the ncu capture of the x-face flux kernel on the 192x96x64 torus
 # (profiles/k_flux_x_torus_192x96x64.md): FP64 operations per face (DADD +
-# DMUL + 2 DFMA thread instructions / faces).  That capture's DRAM bytes
-# (971 MB per launch, mostly register spill) belong to the build before the
-# magnetic floor moved to k_flux_fix, which cut the spills; the current
-# build's traffic has not been captured, so the line reports none.
-FLUX_FP64_PER_FACE = 1895.5
+# DMUL + 2 DFMA thread instructions / faces), and the DRAM bytes of a launch.
+FLUX_FP64_PER_FACE = 1884.6
+FLUX_TRAFFIC = {"shape": (192, 96, 64), "bytes": 313.6e6}
 
 
 def flux_launch(prof, nx, ny, nz):
@@ -107,16 +105,17 @@ def flux_roofline(prof, nx, ny, nz, hbm_peak, peak_src, fp64_peak):
     name, flux_ms, nfaces = flux_launch(prof, nx, ny, nz)
     flux_gbs = 16 * 9 * nfaces / (flux_ms / 1e3) / 1e9 if flux_ms > 0 else None
     tflops = FLUX_FP64_PER_FACE * nfaces / (flux_ms / 1e3) / 1e12 if flux_ms > 0 else None
+    captured = name == "k_flux_x" and (nx, ny, nz) == FLUX_TRAFFIC["shape"]
     return {"kernel": name, "bound": "hbm", "achieved": flux_gbs, "peak": hbm_peak, "unit": "GB/s",
             "frac": (flux_gbs / hbm_peak) if flux_gbs else None,
-            "traffic": None,
-            "traffic_source": "not captured for this build (the previous build's 971 MB per launch was "
-                              "register spill; deferring the magnetic floor cut the spill loads 4.5x)",
+            "traffic": FLUX_TRAFFIC["bytes"] if captured else None,
+            "traffic_source": "ncu capture of this launch, profiles/k_flux_x_torus_192x96x64.md" if captured else None,
             "peak_source": peak_src, "algorithmic_bytes_per_launch": 16 * 9 * nfaces,
             "fp64": {"achieved_tflops": tflops, "peak_tflops": fp64_peak,
                      "frac": (tflops / fp64_peak) if (tflops and fp64_peak) else None,
                      "flop_per_face": FLUX_FP64_PER_FACE,
-                     "note": "the kernel is FP64-latency bound: 13.1 FLOP per algorithmic byte"}}
+                     "note": "bound by instruction issue (59% of the issue slots, 24 of 32 lanes active) and the "
+                             "latency of its loads, not by HBM: 13.1 FLOP per algorithmic byte"}}
 
 
 def fp64_peak_tflops(k):
@@ -619,15 +618,21 @@ WARM_ATTEMPTS_RADTORUS = 2
 SKIP_RADTORUS = 2
 # the implicit solver of the timed radiative-torus steps
 MAIN_SOLVER = "batched"
-# FP64 work of one residual evaluation of the implicit solve on the torus's
-# own cells, nested MHD inversion included: DADD + DMUL + 2 DFMA thread
-# instructions of the one-thread-per-cell solver over its counted
-# evaluations (ncu capture of the first 262144 cells of the implicit step
-# after 3 time steps, profiles/k_rad_plain_fp64_per_evaluation.md)
-IMP_FP64_PER_EVAL = 2884.5
+# FP64 work of the implicit solve per evaluation its counters count, on the
+# torus's own cells: DADD + DMUL + 2 DFMA thread instructions of the
+# one-lane-a-cell solver over its counted evaluations (ncu capture of the first
+# 262144 cells of the implicit step after 3 time steps,
+# profiles/k_rad_plain_fp64_per_evaluation.md).  The counters count the
+# evaluations of the reference's sequence; the ones that need no computation
+# (the final inversion, a base evaluation after a trial on gas primitives) are
+# in the quotient's denominator and not in its numerator.
+IMP_FP64_PER_EVAL = 2122.1
 # the same figure on the batched-solve cells (the first 65536 of the 2^22,
-# seed 2026; profiles/k_rad_plain_fp64_per_evaluation.md)
-IMP_FP64_PER_EVAL_CELLS = 2838.5
+# seed 2026)
+IMP_FP64_PER_EVAL_CELLS = 2200.1
+IMP_WORK = ("FP64 operations of the one-lane-a-cell form on the same kind of cells, per evaluation of the reference's "
+            "sequence; the four-lane kernel repeats some in all four lanes (not counted) and skips trials that their "
+            "energy rejects (counted)")
 
 CPU_REF_CHILD = r"""
 import json, sys, time
@@ -846,7 +851,7 @@ def our_arm_radtorus(args, wl, rank, world, local_rank):
             "share_of_step": solve_ms / total if total else None}
     if IMP_FP64_PER_EVAL and solve_ms > 0:
         tf = IMP_FP64_PER_EVAL * c_prof["imp_evals"] / (solve_ms / 1e3) / 1e12
-        roof.update(achieved=tf, frac=tf / fp64_peak, flop_per_evaluation=IMP_FP64_PER_EVAL)
+        roof.update(achieved=tf, frac=tf / fp64_peak, flop_per_evaluation=IMP_FP64_PER_EVAL, work=IMP_WORK)
     else:
         roof.update(achieved=None, frac=None)
     it_main = c_main["imp_iters"] / max(1, c_main["imp_solves"])
@@ -1150,7 +1155,7 @@ def our_arm_radcells(args, wl, rank, world, local_rank):
                      "peak_source": "measured live (DMUL+DADD chains, no FMA)", "achieved": tf,
                      "frac": tf / fp64_peak if tf else None, "traffic": None, "evaluations": int(stats[3]),
                      "solve_ms": ms_one,
-                     "flop_per_evaluation": IMP_FP64_PER_EVAL_CELLS},
+                     "flop_per_evaluation": IMP_FP64_PER_EVAL_CELLS, "work": IMP_WORK},
         "e2e": {"value": e2e_value, "unit": RAD_UNIT, "h2d_bytes_per_step": n * (13 + 13 + 20 + 20 + 1) * 8,
                 "d2h_bytes_per_step": n * (26 * 8 + 12)},
         "gpu_launches": launches * args.steps,
