@@ -220,10 +220,11 @@ int kgpu_get_counters(kgpu_ctx *ctx, unsigned long long out[4]);
  * pass, cells handed to the entropy equation; with radiation: [8] M1
  * inversions corrected (U2PRAD fixup requests), [9] implicit solves where
  * every attempt failed (RADIMP fixups), [10] their Newton iterations over
- * all attempts, [11] passes of the batched solver with work, [12] warm-start
- * fallbacks, [13] residual evaluations of the implicit solves, [14] Newton
- * steps of the MHD inversions nested in those evaluations, [15] their
- * W-function evaluations, [16] evaluations whose nested inversion went over
+ * all attempts, [11] resident launches of the solver with work, [12] warm-
+ * start fallbacks, [13] residual evaluations of the reference's sequence (those
+ * the solver need not compute again are counted too), [14] Newton steps of the
+ * MHD inversions nested in those evaluations, [15] W-function evaluations that
+ * single lanes made in them, [16] evaluations whose nested inversion went over
  * its per-lane cap and was handed to a whole warp, [17] implicit solves,
  * [18] cells where the radiation floors acted; [19] faces where a side's
  * reconstructed state needed the magnetic floor.  Returns how many were
@@ -428,7 +429,8 @@ int kgpu_rad_implicit_cells(int n, const kgpu_rad_params *rp, const double *uu, 
                             int *attempt, int *iters, int mode);
 /* The same on device pointers, asynchronously on `stream` (a cudaStream_t,
  * or null for the default stream).  stats, when not null, receives after
- * completion: [0] Newton iterations over all attempts, [1] passes run.
+ * completion: [0] Newton iterations over all attempts, [1] resident launches
+ * with work.
  * Temporary device memory of the batched and persistent variants is taken
  * from `work`, which must hold kgpu_rad_work_bytes(n) bytes (null for the
  * plain one). */
@@ -443,7 +445,7 @@ int kgpu_rad_implicit_cells_device(int n, const kgpu_rad_params *rp, const doubl
  * the cells' features); where that attempt fails it is repeated from the
  * cell's own guess and the reference cascade follows, so every cell still
  * converges to RADIMPCONV or fails as the reference would.  stats: [0]
- * Newton iterations over all attempts, [1] passes, [2] cells whose warm
+ * Newton iterations over all attempts, [1] launches, [2] cells whose warm
  * attempt failed (fallbacks). */
 int kgpu_rad_implicit_cells_warm_device(int n, const kgpu_rad_params *rp, const double *uu, const double *pp,
                                         const double *g, const double *G, const double *dt, const float *ypred,

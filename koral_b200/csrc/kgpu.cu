@@ -6,12 +6,13 @@
 // metric tables are [component][point]; with an axisymmetric metric only one
 // phi slice is stored, which keeps them L2-resident.
 //
-// One explicit operator (op_explicit, finite.c:646-1234) is four launches:
+// One explicit operator (op_explicit, finite.c:646-1234) is these launches:
 //   k_wavespeeds  cell speeds of loop_1 + the CFL maximum (atomic on bits)
 //   k_flux<d>     per face: reconstruction of both sides, floors, fluxes,
 //                 p2u of both states and the LLF/HLL combination, fused; the
 //                 reference's face-state and one-sided-flux arrays never
-//                 reach HBM
+//                 reach HBM (small grids: all directions in k_flux_all)
+//   k_flux_fix_all  the faces whose states need the magnetic floor
 //   k_emf         corner EMFs of flux-CT (magn.c:199-297)
 //   k_update      metric source terms and the unsplit update; the
 //                 magnetic-field fluxes that flux_ct() rewrites are formed
@@ -470,12 +471,12 @@ __global__ void k_wavespeeds(Grid G, Box b) {
 // conserved values with shuffles and each lane stores every other variable.
 // Per face the arithmetic is exactly that of the one-thread form.
 // blocks per SM the face-flux, update and first inversion kernels are
-// compiled for (registers per thread = 65536 / (128 x this)); they are
-// FP64-latency bound, so occupancy is traded against spills (measured on the
-// 192x96x64 torus, x faces: 0.66 ms at 4 blocks, 128 registers without DRAM
-// spill traffic; 0.558 ms at 5 blocks, 96 registers; 0.538 ms at 6, 80
-// registers; 0.525 ms at 7, 72 registers; 0.56 ms at 8 blocks, 64
-// registers, whose spills then reach DRAM: 1.2 GB written per launch)
+// compiled for (registers per thread = 65536 / (128 x this)): more resident
+// warps hide the latency of loads and FP64 instructions, against spills.  The
+// lines were drawn on the x faces of the 192x96x64 torus with the magnetic
+// floor inline: 0.66 ms at 4 blocks, 0.558 at 5, 0.538 at 6, 0.525 at 7, 0.56
+// at 8, whose spills then reached DRAM.  Since the floor left the kernels 7
+// blocks take 0.357 ms; the autotuner looks at the others
 #ifndef KGPU_FLUX_MIN_BLOCKS
 #define KGPU_FLUX_MIN_BLOCKS 7
 #endif

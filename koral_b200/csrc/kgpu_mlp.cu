@@ -1,4 +1,4 @@
-// The warm-start network: a 16 -> 128 -> 128 -> 5 multilayer perceptron with
+// The warm-start network: a 16 -> 128 -> 128 -> 7 multilayer perceptron with
 // SiLU activations, BF16 weights and activations and FP32 accumulation on
 // the tensor cores (mma.sync m16n8k16), trained on the device by the
 // kernels below (forward, backward, Adam) and evaluated on the device to
@@ -35,7 +35,7 @@ namespace {
 typedef __nv_bfloat16 bf16;
 
 // FP32 parameter blob: W1[16][128], b1[128], W2[128][128], b2[128],
-// W3[128][8] (outputs 5..7 unused, kept zero), b3[8]; then the output
+// W3[128][8] (output 7 unused, kept zero), b3[8]; then the output
 // standardisation mean[8], scale[8].
 constexpr int OW1 = 0;
 constexpr int OB1 = OW1 + MLP_IN * MLP_H;

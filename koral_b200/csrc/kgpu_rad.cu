@@ -34,10 +34,6 @@ using namespace kgpu;
 #ifndef KGPU_RAD_MIN_BLOCKS
 #define KGPU_RAD_MIN_BLOCKS 4
 #endif
-// default of kgpu_rad_solver_opts.tail
-#ifndef KGPU_RAD_TAIL_BLOCKS
-#define KGPU_RAD_TAIL_BLOCKS 8
-#endif
 
 int kgpu_report_cuda(const char *what, cudaError_t e);   // kgpu.cu: records the error for kgpu_last_error
 
@@ -68,14 +64,14 @@ RadParams to_dev(const kgpu_rad_params &p) {
 
 // Tuning of the batched and persistent forms (kgpu_rad_solver_opts)
 struct Opts {
-  int pass_iters = 4;       // kept for callers that set it: the batched form has no passes any more
+  int pass_iters = 4;       // pass_iters, tail and hard: kept for callers that set them, read by nothing
   int inner_cap = 64;       // W-function evaluations of a nested inversion in one lane (0: no cap)
-  int tail = KGPU_RAD_TAIL_BLOCKS;   // kept likewise (it sized a tail of the passes)
+  int tail = 8;
   int warm_attempts = IMP_NATTEMPTS;
   int thin = 8;             // persistent: hand-off threshold of live lanes once the list is empty
   int blocks_per_sm = 0;    // persistent: resident blocks per SM (0: occupancy limit)
   int skip = 1;             // warm start: begin with the attempt the network expects to succeed
-  int hard = 16;            // kept likewise (it routed cells to that tail)
+  int hard = 16;
 };
 Opts g_opts;   // the context-free entry points' values
 
@@ -120,7 +116,8 @@ struct Cell {
   int *status, *attempt, *iters;
 };
 
-// work area of the batched form (all device memory carved from one block)
+// work area of the batched and persistent forms (all device memory carved
+// from one block)
 struct Work {
   double *wpp;      // [n][13] iterate of the running attempt
   int *wit;         // [n] its iteration count
@@ -130,7 +127,7 @@ struct Work {
   double *wguess;   // [n][13] the predicted iterate (warm start only)
   int *q[2][2];     // queues of cell indices (persistent form)
   int *count;       // [kCounters]
-  int *qs;          // cooperative queue of the current pass: cell indices ...
+  int *qs;          // hand-over queue (persistent form): cell indices ...
   ImpState *ss;     // ... and the states of their interrupted evaluations
   int nslots;       // its capacity
   unsigned long long *stats;  // [0] Newton iterations, [1] resident launches, [2] fallbacks of the warm start,
@@ -142,7 +139,7 @@ struct Work {
 };
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-// capacity of the cooperative queue: an eighth of the cells (a cell that
+// capacity of the hand-over queue: an eighth of the cells (a cell that
 // finds the queue full carries on alone, without the cap)
 inline int slow_slots(int n) { return n / 8 > 1024 ? n / 8 : 1024; }
 
@@ -306,9 +303,9 @@ __device__ inline int warp_slot(int *qcount, bool pred) {
   return pred ? base + __popc(bits & ((1u << lane) - 1u)) : -1;
 }
 
-// Start of the batched form: every cell's cascade state (first attempt,
-// no iteration yet, the guess as iterate), queued by the primitives its
-// first attempt works on, so that warps of a pass run one kind of inversion.
+// Start of the batched and persistent forms: every cell's cascade state
+// (first attempt, no iteration yet, the guess as iterate), queued by the kind
+// of its first attempt, so that a warp's cells run one kind of inversion.
 // gate >= 0: only cells whose previous solve (the attempt and iteration
 // outputs, read before this solve overwrites them) needed a later attempt
 // or more than gate Newton iterations start from the prediction
@@ -1041,13 +1038,12 @@ __global__ void __launch_bounds__(128, KGPU_RAD_MIN_BLOCKS) k_rad_persist(RadPar
 // k_rad_finish: the cells k_rad_persist handed over, each run to its end by
 // a whole warp that takes them from a counter.  At the start of every
 // Newton iteration lanes 0..8 evaluate the base and the Jacobian columns on
-// both sides together (imp_eval_entry, as k_rad_tail does), each with the
-// cap on its nested inversion; the entries that ran over the cap, and the
-// remaining evaluations (damped trials, the final inversion, and the
-// evaluation a handed-over state stopped in), run their nested MHD
-// inversion with all 32 lanes (the damped trials tried 32 at a time, as
-// k_rad_slow does).  The sequence of operations per cell is that of the
-// one-thread form.
+// both sides together (imp_eval_entry), each with the cap on its nested
+// inversion.  The entries that ran over the cap, and the remaining evaluations
+// (damped trials, and the one a handed-over state stopped in), run their
+// nested MHD inversion with all 32 lanes, the damped points of a step tried 32
+// at a time.  The sequence of operations per cell is that of the one-thread
+// form.
 __global__ void __launch_bounds__(128, KGPU_RAD_MIN_BLOCKS) k_rad_finish(RadParams R, Cell C, Work W, int warm_attempts,
                                                     unsigned inner_cap) {
   const unsigned FULL = 0xffffffffu;
@@ -1237,7 +1233,7 @@ extern "C" int kgpu_rad_set_inner_cap(int cap) {
 }
 
 extern "C" int kgpu_rad_set_tail(int on) {
-  g_opts.tail = on ? KGPU_RAD_TAIL_BLOCKS : 0;
+  g_opts.tail = on ? Opts().tail : 0;
   return 0;
 }
 
@@ -1268,7 +1264,7 @@ static long long solve_launches(int mode) {
 }
 
 // acc (device, optional): counters the solve adds to instead of reporting
-// through stats: [0] Newton iterations, [1] passes with work, [2] warm-start
+// through stats: [0] Newton iterations, [1] resident launches with work, [2] warm-start
 // fallbacks, [3] residual evaluations, [4] nested Newton steps, [5] their
 // W-function evaluations, [6] evaluations handed to a whole warp.
 // Launches only (no allocation, no synchronisation) when stats is null, so

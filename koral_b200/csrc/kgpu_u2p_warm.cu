@@ -16,9 +16,8 @@
 // invert is never smaller than the reference's.  Every Newton step is the
 // unchanged FP64 one and ends on the same residual test (U2PCONV).
 //
-// Without a prediction the kernel is the reference's u2p itself (the same
-// function as kgpu_u2p_cells, same bits), with its Newton iterations
-// counted.
+// Without a prediction it is the reference's u2p itself (the bits of
+// kgpu_u2p_cells), with its Newton iterations counted, in two launches.
 #include <cuda_runtime.h>
 #include <string.h>
 
@@ -318,20 +317,18 @@ __global__ void k_u2p_warm_cells(U2PParams P, int n, int nv, const double *uu, d
       u[iv] = uu[(long)i * nv + iv];
       p[iv] = p0[iv] = pp[(long)i * nv + iv];
     }
-    int fix = 0, ret;
-    {
-      const float *y = ypred + (long)i * MLP_OUTP;
-      // a predicted change of W smaller than wgate is within the network's
-      // own error: the guess's W is kept; the energy equation is skipped
-      // where the score passes sgate
-      const double W0 = fabsf(y[0]) >= wgate ? u2p_warm_w(G.gamma, p0, g, y[0]) : u2p_initial_w(G.gamma, p0, g);
-      ret = W0 > 0. ? u2p_counted(G, u, p, g, fix, W0, y[1] > sgate, it, fe) : -3;
-      if (ret < -1) {
-        // fallback: the reference's inversion from the reference's guess
-        fell = 1;
-        for (int iv = 0; iv < NVMAX; iv++) p[iv] = p0[iv];
-        ret = u2p_counted(G, u, p, g, fix, -1., false, it, fe);
-      }
+    int fix = 0;
+    const float *y = ypred + (long)i * MLP_OUTP;
+    // a predicted change of W smaller than wgate is within the network's
+    // own error: the guess's W is kept; the energy equation is skipped
+    // where the score passes sgate
+    const double W0 = fabsf(y[0]) >= wgate ? u2p_warm_w(G.gamma, p0, g, y[0]) : u2p_initial_w(G.gamma, p0, g);
+    int ret = W0 > 0. ? u2p_counted(G, u, p, g, fix, W0, y[1] > sgate, it, fe) : -3;
+    if (ret < -1) {
+      // fallback: the reference's inversion from the reference's guess
+      fell = 1;
+      for (int iv = 0; iv < NVMAX; iv++) p[iv] = p0[iv];
+      ret = u2p_counted(G, u, p, g, fix, -1., false, it, fe);
     }
     for (int iv = 0; iv < NVMAX; iv++) pp[(long)i * nv + iv] = p[iv];
     status[i] = ret;
@@ -476,7 +473,9 @@ extern "C" int kgpu_u2p_cells_device(int n, const kgpu_config *cfg, int nv, cons
     if (e == cudaSuccess) {
       // a range per block: as many blocks as two per SM hold, so that a
       // block's few hard cells fill more of its lanes, down to a range of 128
-      int range = (n + 2 * 148 - 1) / (2 * 148);
+      int dev = 0, sms = 148;
+      if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      int range = (n + 2 * sms - 1) / (2 * sms);
       range = range < REST_THREADS ? REST_THREADS : (range > REST_RANGE ? REST_RANGE : range);
       k_u2p_rest<<<(n + range - 1) / range, REST_THREADS, 0, s>>>(P, n, nv, range, uu, pp, g, G, status, fixup, iters,
                                                                    dstats);
