@@ -110,14 +110,12 @@ def test_rad_implicit_matches_reference(kgpu, ref, cells):
 
 
 def test_rad_batched_equals_plain(kgpu, cells):
-    """The work-queue forms resume each Newton solve exactly where it paused:
-    their results are those of the one-thread-per-cell form, bit for bit.
-    Batched: any number of iterations per pass, with the warp-per-cell tail
-    (the base and Jacobian evaluations of an iteration done by lanes
-    together) and without it.  Persistent: any hand-off threshold of a
-    thinned warp, with and without the cap on nested inversions, at one
-    block per SM and at the occupancy limit.  The tuning is passed per call;
-    the process-wide values are not touched."""
+    """The batched and the persistent form do the evaluations of the
+    one-thread-per-cell form and give its results, bit for bit.  Batched: any
+    cap on the evaluations of a nested inversion in one lane (0: none).
+    Persistent: any hand-off threshold of a thinned warp, with and without the
+    cap, at one block per SM and at the occupancy limit.  The tuning is passed
+    per call; the process-wide values are not touched."""
     import torch
     rp, uu, pp, g, G, dt = cells
     d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (uu, pp, g, G, dt)]
@@ -125,7 +123,7 @@ def test_rad_batched_equals_plain(kgpu, cells):
     host = kgpu.rad_implicit_cells(rp, uu, pp, g, G, dt, mode=kgpu.RAD_PLAIN)
     for x, y in zip(a, host):
         assert np.array_equal(x, y)
-    variants = [(kgpu.RAD_BATCHED, dict(tail=tail, pass_iters=k)) for tail in (16, 1, 0) for k in (1, 3, 8)]
+    variants = [(kgpu.RAD_BATCHED, dict(inner_cap=cap)) for cap in (64, 16, 4, 1, 0)]
     variants += [(kgpu.RAD_PERSISTENT, dict(thin=thin, inner_cap=cap, blocks_per_sm=b))
                  for thin, cap, b in ((8, 64, 0), (0, 64, 0), (32, 64, 1), (8, 0, 0), (16, 4, 1))]
     stats = {}

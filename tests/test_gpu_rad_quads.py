@@ -1,7 +1,9 @@
 """The batched implicit solve (four lanes a cell, work lists by kind of
 attempt) against the other forms, bit for bit, at the sizes where its lists
 and its lanes can go wrong: fewer cells than a warp takes, one cell a warp,
-the last warp part-filled, and enough cells that every quad takes several.
+the last warp part-filled, as many cells as the chip holds warps and one more
+(where the warps of a block begin to go in step), and enough cells that every
+quad takes several.
 
 * From the cells' own guess: the one-thread-per-cell form, results and the
   counters of Newton iterations and evaluations, whatever the cap on the
@@ -34,7 +36,7 @@ def assert_same(a, b):
 
 
 @pytest.mark.parametrize("sigma", [None, SIGMA])
-@pytest.mark.parametrize("n", [1, 3, 33, 1201, 21001])
+@pytest.mark.parametrize("n", [1, 3, 33, 1201, 2368, 2369, 21001])
 def test_quads_equal_plain(kgpu, n, sigma):
     rp, d = device_cells(kgpu, n, sigma)
     a = kgpu.rad_solve_device(rp, *d, mode=kgpu.RAD_PLAIN, nstats=7)

@@ -25,8 +25,8 @@ Parity policy.
    L1 difference the reference itself shows when one input variable of every
    cell is nudged by one ulp (five nudges: gas energy up and down,
    radiation energy up and down, density up), times two.
- - solver variants: the batched and the one-thread-per-cell solvers, and a
-   stream and a CUDA-graph replay of the step, give the same bits.
+ - solver variants (same bits from every solver form, from the stream and from
+   a CUDA graph): test_gpu_solver_forms.py, which needs no reference build.
 """
 import ctypes
 import os
@@ -173,62 +173,6 @@ def test_radtorus_op_implicit_within_reference_sensitivity(kgpu, oracle, ref_aft
     # solves where every attempt failed (RADIMP fixups): a few per cent
     print("GPU failed solves:", c["radimp_failed"])
     assert c["radimp_failed"] <= 0.05 * gpu.shape[0]
-
-
-def test_radtorus_solver_variants_and_graph_identical(kgpu, oracle):
-    R = oracle.RefKoral(LIB)
-    R.init()
-    u, p, tsd = R.array("u").copy(), R.array("p").copy(), R.scalar("tstepdenmax")
-    out = []
-    # hard: cells hard in their previous solve start in the tail (0: all that
-    # took more than no iteration, i.e. every cell after the first step; -1: none)
-    for mode, graph, hard in ((kgpu.RAD_BATCHED, False, 16), (kgpu.RAD_BATCHED, True, 16), (kgpu.RAD_PLAIN, True, 16),
-                              (kgpu.RAD_PERSISTENT, False, 16), (kgpu.RAD_PERSISTENT, True, 16),
-                              (kgpu.RAD_BATCHED, True, -1), (kgpu.RAD_BATCHED, True, 0)):
-        s = make_gpu(kgpu, R)
-        s.set_implicit_solver(mode, None)
-        s.set_implicit_options(hard=hard)
-        s.upload_state(u.copy(), p.copy())
-        s.tstepdenmax = tsd
-        s.rk2imex_steps(3, graph=graph)
-        out.append(s.download_state())
-        s.close()
-    for k in range(1, len(out)):
-        assert np.array_equal(out[0][0], out[k][0]) and np.array_equal(out[0][1], out[k][1]), k
-
-
-def test_radtorus_solver_options_per_context(kgpu, oracle):
-    """Two contexts in one process hold their own solver tuning: setting one
-    leaves the other alone, a captured step graph is re-captured when its
-    context's options change (its launch count follows them), and the
-    results stay the same bits."""
-    R = oracle.RefKoral(LIB)
-    R.init()
-    u, p, tsd = R.array("u").copy(), R.array("p").copy(), R.scalar("tstepdenmax")
-    a, b = make_gpu(kgpu, R), make_gpu(kgpu, R)
-    for s in (a, b):
-        s.set_implicit_solver(kgpu.RAD_BATCHED, None)
-        s.upload_state(u.copy(), p.copy())
-        s.tstepdenmax = tsd
-    a.set_implicit_options(pass_iters=1)
-    assert b.implicit_options().pass_iters == kgpu.solver_opts().pass_iters and a.implicit_options().pass_iters == 1
-    la = a.launches
-    a.rk2imex_steps(1, graph=True)
-    la = a.launches - la
-    lb = b.launches
-    b.rk2imex_steps(1, graph=True)
-    lb = b.launches - lb
-    assert la > lb   # one Newton iteration per pass: more pass launches
-    b.set_implicit_options(pass_iters=1)   # between two graph steps: re-captured
-    lb2 = b.launches
-    b.rk2imex_steps(1, graph=True)
-    assert b.launches - lb2 == la
-    a.rk2imex_steps(1, graph=True)
-    ua, pa = a.download_state()
-    ub, pb = b.download_state()
-    assert np.array_equal(ua, ub) and np.array_equal(pa, pb)
-    with pytest.raises(kgpu.KgpuError):
-        a.set_implicit_options(thin=33)
 
 
 def test_radtorus_two_steps_within_reference_sensitivity(kgpu, oracle, tmp_path):

@@ -10,8 +10,9 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("far", [0.02, 1.0, 6.0])
-@pytest.mark.parametrize("n", [1, 31, 129, 4097, 40001])
+# 310001: ranges of the largest size, 1024 cells, and a last one that is not full
+@pytest.mark.parametrize("n, far", [(n, far) for n in (1, 31, 129, 4097, 40001) for far in (0.02, 1.0, 6.0)] +
+                         [(310001, 1.0)])
 def test_device_cells_equal_one_thread_per_cell(kgpu, n, far):
     import torch
     rp = kgpu.rad_params()
